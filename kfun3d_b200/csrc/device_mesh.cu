@@ -310,7 +310,8 @@ void kf_ilu_release(DevMesh &m);
 void kf_free_packed(PackedSweep pk[2])
 {
   for (int s = 0; s < 2; s++) {
-    void *ptrs[] = {pk[s].row, pk[s].first, pk[s].col, pk[s].src, pk[s].chunk[0], pk[s].chunk[1]};
+    void *ptrs[] = {pk[s].row,      pk[s].first,    pk[s].col,      pk[s].src,
+                    pk[s].chunk[0], pk[s].chunk[1], pk[s].chunk[2], pk[s].slot};
     for (void *q : ptrs)
       if (q) cudaFree(q);
     pk[s] = PackedSweep{};
@@ -321,9 +322,10 @@ void kf_free_packed(PackedSweep pk[2])
 // lower sweep contributes its lower blocks [d.y, d.z) (matrix/sptrsv.cpp:173-189
 // reads them in this column order); slot s of the upper sweep its inverted
 // diagonal block and then its upper blocks [d.y, d.z) (matrix/sptrsv.cpp:191-209).
-// Each level's slots are cut into chunks, one CTA each, twice: at most 32 rows
-// and 256 blocks, and at most 64 rows and 512 blocks.  KFUN3D_ERR_ARG (and
-// nothing allocated) when a row has more than KF_PK_ROW_MAX blocks.
+// Each level's slots are cut into chunks three times: at most 32 rows and 256
+// blocks, at most 64 rows and 512 blocks (one CTA each), and for the
+// data-flow sweeps 4 rows and 40 blocks (8 lanes a row) or 8 rows and 64
+// blocks (4 lanes; one warp each).  KFUN3D_ERR_ARG (and nothing allocated) when a row has more than KF_PK_ROW_MAX blocks.
 // (f(i) for every i in [0, n), interleaved over the host's threads: for
 // items of uneven size, such as levels)
 template <class F> static void parallel_items(size_t n, size_t work, F f)
@@ -366,7 +368,8 @@ void kf_level_descriptors(const HostPattern &p, std::vector<uint4> &dl, std::vec
 
 int kf_build_packed(PackedSweep pk[2], const HostPattern &p, const std::vector<uint4> &desc_l,
                     const std::vector<uint4> &desc_u, const uint4 *ddesc_l, const uint4 *ddesc_u,
-                    const uint32_t *ja, const uint32_t *diag, cudaStream_t st)
+                    const uint32_t *ja, const uint32_t *diag, const uint32_t *row_node, int flow_lanes,
+                    cudaStream_t st)
 {
   const size_t N = p.n;
   for (int sw = 0; sw < 2; sw++) {
@@ -387,12 +390,16 @@ int kf_build_packed(PackedSweep pk[2], const HostPattern &p, const std::vector<u
     // the streams (slot rows, block columns, source blocks) written on the device
     bool ok = upload(&o.first, first.data(), N + 1) == cudaSuccess &&
               cudaMalloc(&o.row, std::max<size_t>(N, 1) * sizeof(uint32_t)) == cudaSuccess &&
-              cudaMalloc(&o.col, std::max<size_t>(nblk, 1) * sizeof(uint32_t)) == cudaSuccess &&
+              // (bulk copies of a chunk's columns are widened to 4-entry boundaries)
+              cudaMalloc(&o.col, (nblk + 4) * sizeof(uint32_t)) == cudaSuccess &&
+              cudaMemsetAsync(o.col, 0, (nblk + 4) * sizeof(uint32_t), st) == cudaSuccess &&
+              cudaMalloc(&o.slot, std::max<size_t>(N, 1) * sizeof(uint4)) == cudaSuccess &&
               cudaMalloc(&o.src, std::max<size_t>(nblk, 1) * sizeof(uint32_t)) == cudaSuccess;
-    ok = ok && kf_packed_streams_device((uint32_t)N, sw == 1, sw == 0 ? ddesc_l : ddesc_u, o.first, ja, diag, o.row,
-                                        o.col, o.src, st) == KFUN3D_OK;
-    for (int cut = 0; cut < 2 && ok; cut++) {
-      const uint32_t rows = cut == 0 ? 32u : 64u, budget = 8u * rows;
+    ok = ok && kf_packed_streams_device((uint32_t)N, sw == 1, sw == 0 ? ddesc_l : ddesc_u, o.first, ja, diag, row_node,
+                                        o.row, o.col, o.src, o.slot, st) == KFUN3D_OK;
+    for (int cut = 0; cut < 3 && ok; cut++) {
+      const uint32_t rows = cut == 0 ? 32u : cut == 1 ? 64u : 32u / (uint32_t)flow_lanes;
+      const uint32_t budget = cut == 2 ? (flow_lanes == 8 ? 40u : 64u) : 8u * rows;
       std::vector<uint4> chunk;
       std::vector<uint32_t> lev(1, 0);
       uint32_t maxblk = 0;
@@ -427,7 +434,8 @@ static void release_device(MatrixHandle *h)
   if (!m) return;
   kf_ilu_release(*m);   // the spatial ILU set's arrays; the reference set's fields are back in place
   kf_free_packed(m->iset[0].pk);
-  if (m->pk_buf) cudaFree(m->pk_buf);
+  for (void *p : {m->pk_buf, (void *)m->flow_buf, (void *)m->flow_ctl})
+    if (p) cudaFree(p);
   void *ptrs[] = {m->col, m->egeo, m->xyz, m->inc_ptr, m->inc_oth, m->inc_edge, m->inc_blk, m->inc_w, m->wf_nodes,
                   m->wf_n, m->s_n, m->f_n, m->bnd_of, m->bnd_node, m->bnd_ptr, m->bnd_ent, m->ia, m->ja,
                   m->diag, m->tblk, m->lpos, m->last_lower, m->lev_l, m->lev_u, m->A, m->lslot, m->dinv,
@@ -560,6 +568,13 @@ static int lists_match_host(const DevMesh &m, const GEOMETRY *g, const HostPatte
     return -1;
   }
   return same ? 1 : 0;
+}
+
+cudaError_t kf_flow_reset(DevMesh &m)
+{
+  cudaError_t e = cudaMemsetAsync(m.flow_buf, 0xff, 3 * 4 * (size_t)m.N * sizeof(double), m.stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m.flow_ctl, 0, 4 * sizeof(unsigned), m.stream);
+  return e;
 }
 
 extern "C" long kfun3d_device_query(const GEOMETRY *g, const char *key)
@@ -875,8 +890,17 @@ DevMesh *kf_device(const GEOMETRY *g)
     // the packed factor (room for FP64 blocks, shared by both ILU orders) and
     // this pattern's packed level schedule
     KF_CUDA(cudaMalloc(&m->pk_buf, 16 * (size_t)m->nnz * sizeof(double)));
+    KF_CUDA(cudaMalloc(&m->flow_buf, 3 * dofs * sizeof(double)));
+    KF_CUDA(cudaMalloc(&m->flow_ctl, 4 * sizeof(unsigned)));
+    KF_CUDA(kf_flow_reset(*m));
+    // lanes per row of the data-flow sweeps: eight halve a row's chain of
+    // products, which is what small meshes wait for; four keep twice the rows
+    // in flight, which is what fills the machine on large ones (measured, 8 /
+    // 4 lanes: 25^3 72 / 83 us, 40^3 81 / 95, 70^3 229 / 217, 120^3 724 / 630)
+    m->flow_lanes = N < 150000u ? 8 : 4;
     // ERR_ARG: rows too long, no packed schedule
-    const int pkrc = kf_build_packed(m->iset[0].pk, p, dl, du, m->desc_l, m->desc_u, m->ja, m->diag, m->stream);
+    const int pkrc = kf_build_packed(m->iset[0].pk, p, dl, du, m->desc_l, m->desc_u, m->ja, m->diag, nullptr,
+                                     m->flow_lanes, m->stream);
     if (pkrc == KFUN3D_ERR_CUDA) {
       kf_set_error(KFUN3D_ERR_CUDA, "device mirror: building the packed triangular-solve schedule failed");
       return nullptr;
@@ -892,10 +916,12 @@ DevMesh *kf_device(const GEOMETRY *g)
         m->pk_cut[1] = r32 == 32 ? 0 : 1;
       }
     }
-    // triangular-solve schedule (KFUN3D_SPTRSV): "packed" (default: one
-    // launch per level with programmatic dependent launch, each CTA's rows
-    // one contiguous run of the packed factor staged into shared memory by a
-    // bulk copy), "pdl4" (one launch per level with programmatic dependent
+    // triangular-solve schedule (KFUN3D_SPTRSV): by default both sweeps in one
+    // launch over the packed factor, each row waiting for the values it reads
+    // (k_trsv_flow), or "packed" where a row is too long for it or when named
+    // (one launch per level with programmatic dependent launch, each CTA's
+    // rows one contiguous run of the packed factor staged into shared memory
+    // by a bulk copy), "pdl4" (one launch per level with programmatic dependent
     // launch, 4 lanes per row, blocks read in the matrix's order), "pdl"
     // (the same with 16 lanes per row), "persistent" / "mono" (one
     // cooperative launch, bounded grid barrier between levels), "syncfree"
@@ -910,6 +936,7 @@ DevMesh *kf_device(const GEOMETRY *g)
     if (env && strcmp(env, "mono") == 0) m->trsv_mode = 5;
     if (env && strcmp(env, "pdl4") == 0) m->trsv_mode = 7;
     if (env && strcmp(env, "packed") == 0 && m->iset[0].pk[0].chunk[0]) m->trsv_mode = 8;
+    m->pk_flow = !(env && strcmp(env, "packed") == 0);
     std::vector<uint32_t> lp(p.lev_l_ptr);
     lp.insert(lp.end(), p.lev_u_ptr.begin(), p.lev_u_ptr.end());
     KF_CUDA(upload(&m->lev_ptr_d, lp.data(), lp.size()));

@@ -284,24 +284,25 @@ int build_spatial(DevMesh &m, const GEOMETRY *g)
     lp.insert(lp.end(), p.lev_u_ptr.begin(), p.lev_u_ptr.end());
     up(&s.lev_ptr_d, lp);
   }
+  // the fill's view of the renumbered pattern, per node of the mesh, and
+  // the node of each renumbered row (on the device)
+  up(&m.ilu_rank, rank);
+  if (ok && kf_fill_targets_device(m, s) != KFUN3D_OK) ok = false;
+  tr.mark("fill targets");
   {
     std::vector<uint4> dl, du;
     kf_level_descriptors(p, dl, du);
     up(&s.desc_l, dl);
     up(&s.desc_u, du);
-    if (ok && kf_build_packed(s.pk, p, dl, du, s.desc_l, s.desc_u, s.ja, s.diag, m.stream) == KFUN3D_ERR_CUDA)
+    if (ok && kf_build_packed(s.pk, p, dl, du, s.desc_l, s.desc_u, s.ja, s.diag, s.row_node, m.flow_lanes,
+                              m.stream) == KFUN3D_ERR_CUDA)
       ok = false;
   }
   tr.mark("level descriptors, packed schedule");
-  // the fill's view of the renumbered pattern, per node of the mesh, and
-  // the node of each renumbered row (on the device)
-  up(&m.ilu_rank, rank);
-  if (ok && kf_fill_targets_device(m, s) != KFUN3D_OK) ok = false;
   if (ok && cudaMalloc(&m.pb, 4 * N * sizeof(double)) != cudaSuccess) ok = false;
   if (ok && cudaMalloc(&m.px, 4 * N * sizeof(double)) != cudaSuccess) ok = false;
-  // one launch per level (programmatic dependent launch, each CTA's rows one
-  // contiguous run of the packed factor) by default; KFUN3D_SPTRSV picks
-  // another schedule
+  // the packed factor by default (data-flow sweeps, or one launch per level);
+  // KFUN3D_SPTRSV picks another schedule
   s.trsv_mode = s.pk[0].chunk[0] ? 8 : 7;
   const char *env = getenv("KFUN3D_SPTRSV");
   if (env && strcmp(env, "pdl4") == 0) s.trsv_mode = 7;
@@ -313,7 +314,6 @@ int build_spatial(DevMesh &m, const GEOMETRY *g)
     kf_set_error(KFUN3D_ERR_CUDA, "spatial ILU(0) order: out of device memory");
     return KFUN3D_ERR_CUDA;
   }
-  tr.mark("fill targets");
   s.valid = true;
   return KFUN3D_OK;
 }

@@ -180,17 +180,20 @@ __device__ __forceinline__ bool kf_grid_barrier(unsigned *bar, int *err)
 // one contiguous run of the stream.  The blocks are copied into the stream
 // after every factorisation (k_trsv_pack, through src).
 constexpr uint32_t KF_PK_ROW_MAX = 1536;   // blocks of one row, at most (larger: no packed schedule)
+constexpr uint32_t KF_FLOW_ROW_MAX = 96;   // longest row the data-flow sweeps take (their shared-memory stage)
 struct PackedSweep {
   uint32_t *row = nullptr;     // [N] matrix row of each slot
   uint32_t *first = nullptr;   // [N+1] first streamed block of each slot
   uint32_t *col = nullptr;     // [nblk] column of each streamed block
   uint32_t *src = nullptr;     // [nblk] matrix block copied to each stream position
-  // two cuts of the levels into chunks, [0] of at most 32 rows and 256 blocks
+  uint4 *slot = nullptr;       // [N] per slot: (matrix row, first block, end block, mesh node)
+  // three cuts of the levels into chunks, [0] of at most 32 rows and 256 blocks
   // (one CTA of 128 threads), [1] of at most 64 rows and 512 blocks (256
-  // threads); a row longer than the budget is a chunk of its own
-  uint4 *chunk[2] = {nullptr, nullptr};   // per CTA: (first slot, end slot, first block, end block)
-  std::vector<uint32_t> lev[2];           // first chunk of each level, nlev + 1 entries
-  uint32_t maxblk[2] = {0, 0};            // blocks of the largest chunk
+  // threads), [2] of the rows and blocks of one warp of the data-flow sweeps
+  // (kf_build_packed's flow_lanes); a row longer than the budget is a chunk of its own
+  uint4 *chunk[3] = {nullptr, nullptr, nullptr};   // (first slot, end slot, first block, end block)
+  std::vector<uint32_t> lev[3];           // first chunk of each level, nlev + 1 entries
+  uint32_t maxblk[3] = {0, 0, 0};         // blocks of the largest chunk
   uint32_t nblk = 0;                      // blocks in the stream
 };
 
@@ -219,14 +222,17 @@ struct IluSet {
 void kf_level_descriptors(const HostPattern &p, std::vector<uint4> &desc_l, std::vector<uint4> &desc_u);
 // Builds the packed level schedule of one pattern from its level-slot
 // descriptors (host copies for the chunk cuts, device copies for the
-// streams) and level offsets; ja and diag are the pattern's device arrays.
+// streams) and level offsets; ja and diag are the pattern's device arrays,
+// row_node its rows' mesh nodes (null: the identity); flow_lanes lanes a row
+// in the data-flow sweeps, whose chunks have 32 / flow_lanes rows.
 // KFUN3D_OK, KFUN3D_ERR_ARG (a row too long: no packed schedule) or
 // KFUN3D_ERR_CUDA, with nothing left allocated on error.
 int kf_build_packed(PackedSweep pk[2], const HostPattern &p, const std::vector<uint4> &desc_l,
                     const std::vector<uint4> &desc_u, const uint4 *ddesc_l, const uint4 *ddesc_u,
-                    const uint32_t *ja, const uint32_t *diag, cudaStream_t st);
+                    const uint32_t *ja, const uint32_t *diag, const uint32_t *row_node, int flow_lanes, cudaStream_t st);
 int kf_packed_streams_device(uint32_t N, bool upper, const uint4 *desc, const uint32_t *first, const uint32_t *ja,
-                             const uint32_t *diag, uint32_t *row, uint32_t *col, uint32_t *src, cudaStream_t st);
+                             const uint32_t *diag, const uint32_t *row_node, uint32_t *row, uint32_t *col,
+                             uint32_t *src, uint4 *slot, cudaStream_t st);
 void kf_free_packed(PackedSweep pk[2]);
 
 // The block pattern built on the device (setup_device.cu): the device arrays,
@@ -369,6 +375,12 @@ struct DevMesh {
   int pk_cut[2] = {0, 0};         // chunk cut used with FP64 / FP32 factors (0: 32 rows, 1: 64 rows)
   bool pk_fp64 = false;           // FP64 factors also take the packed schedule (KFUN3D_PK_FP64=1)
   void *pk_buf = nullptr;         // the packed factor: lower stream, then upper stream (FP64 or FP32 blocks)
+  // data-flow sweeps over the packed factor (k_trsv_flow): rows wait for the
+  // values they read instead of for levels
+  bool pk_flow = true;            // used by mode 8 where the rows fit (KFUN3D_SPTRSV=packed: level launches)
+  int flow_lanes = 8;             // lanes per row in the data-flow sweeps (4 or 8)
+  double *flow_buf = nullptr;     // [3][4N] y of the lower sweep, x of this and of the next solve (KF_FLOW_EMPTY where not written)
+  unsigned *flow_ctl = nullptr;   // [0] which x buffer the next solve writes, [1] CTAs done
   int ilu_active = 0;             // 1: the spatial set is active
   uint32_t *ilu_rank = nullptr;   // [N] row of each node in the spatial set
   double *pb = nullptr, *px = nullptr;   // [4N] right-hand side and solution, spatial numbering
@@ -409,6 +421,10 @@ std::vector<uint32_t> kf_partition_rcb(const double *X, const double *Y, const d
 
 void kf_count_launch(unsigned n = 1);
 void kfun3d_reset_launch_count_by(unsigned long long n);   // undo counts taken during graph capture
+
+// Clears the data-flow sweeps' buffers to "not written" (at set-up, and after
+// a wait that gave up).
+cudaError_t kf_flow_reset(DevMesh &m);
 
 // Kernel families, one set per arithmetic mode (kernels_exact.cu, kernels_fast.cu).
 #define KF_DECLARE_KERNELS(NS)                                                          \

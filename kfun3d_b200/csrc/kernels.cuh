@@ -2062,6 +2062,248 @@ __global__ void __launch_bounds__(256, 4) k_trsv_syncfree(uint32_t N, const uint
   }
 }
 
+// ------------------------------------------------------------------ data-flow sweeps over the packed factor
+
+// "Not written yet": the bits every value of the data-flow buffers holds
+// before its row is solved (a NaN; a result that has the same high word, which
+// only a NaN can, is stored as the canonical NaN instead).
+constexpr long long KF_FLOW_EMPTY = -1ll;
+
+// v = the four values at p where `on` (v is left as it is elsewhere)
+__device__ __forceinline__ void ld_flow(double4 &v, const double *p, uint32_t on)
+{
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n @q ld.relaxed.gpu.global.v4.f64 {%0, %1, %2, %3}, [%4];\n}\n"
+               : "+d"(v.x), "+d"(v.y), "+d"(v.z), "+d"(v.w)
+               : "l"(p), "r"(on)
+               : "memory");
+}
+__device__ __forceinline__ double ld_flow1(const double *p)
+{
+  double v;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_flow(double *p, double v)
+{
+  if (__double2hiint(v) == -1) v = __longlong_as_double(0x7ff8000000000000ll);
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ bool flow_ready(const double4 &v)
+{
+  return __double2hiint(v.x) != -1 && __double2hiint(v.y) != -1 && __double2hiint(v.z) != -1 &&
+         __double2hiint(v.w) != -1;
+}
+
+struct FlowSweep {
+  const uint4 *chunk;    // (first slot, end slot, first block, end block), level after level
+  const uint4 *slot;     // (row, first block, end block, node)
+  const uint32_t *col;   // column of each streamed block
+  const void *pk;        // the sweep's packed blocks
+  uint32_t nc;           // chunks
+};
+
+// Both triangular sweeps (matrix/sptrsv.cpp:34-73) in one cooperative launch
+// without levels: a chunk is up to KF_FLOW_ROWS rows of one level (four lanes
+// per row, lane r = component r) and belongs to one warp; warp w of W works
+// chunks w, w + W, ... of the lower sweep and then of the upper sweep, in that
+// order.  A row polls the very values it reads -- y (lower) or x (upper) of
+// its columns -- until each of them has been written: a value is its own flag
+// (KF_FLOW_EMPTY before), so a level costs one store and one load through L2
+// instead of a grid's completion and the next grid's start.  Values are read
+// and written with relaxed device-scope accesses of 64 bits, and nothing else
+// is communicated.
+//
+// While a chunk is worked, the warp's next chunk is on its way: its blocks and
+// columns, one contiguous run each, come by bulk copies into the warp's other
+// shared-memory stage (mbarrier, bounded wait), its slots into registers.
+//
+// Progress: every CTA is resident (cooperative launch), and a warp waits only
+// for rows of earlier chunks, whose warps work theirs in order.  A wait that
+// gives up sets *err; the warp then runs through its remaining chunks without
+// waiting, so that no copy is left in flight.
+//
+// Buffers: y and the x of this solve must be KF_FLOW_EMPTY on entry.  The upper
+// sweep's row clears its y once it has every x it reads (the rows that read
+// this y are the rows of its upper columns, the pattern being symmetric, and
+// they wrote their x after reading it), and the lower sweep's row clears the x
+// buffer of the next solve; ctl[0] picks the buffer and flips at the end.
+// Arithmetic per row: k_trsv_packed's (each block product summed from zero,
+// subtracted in column order), so the results are the same bit for bit.
+//
+// G lanes per row: quad jj of the row takes columns jj, jj + G/4, ... (P of
+// them at a time), and the products are subtracted in column order through
+// shuffles.  What bounds it: on small meshes the chain of levels, each one
+// store-to-load hop through L2 (0.25 to 0.5 us between two SMs) and one row's
+// products; on large ones the rows in flight, limited by the shared-memory
+// stages (FP64) and registers (FP32), times a chunk's latency (L2 gathers
+// under load, then its instructions; issue slots 37 % busy at 70^3).  One
+// solve, both sweeps, before (level launches) and now: 10^3 FP64 124 -> 50 us,
+// 25^3 FP64 199 -> 72, 40^3 FP32 spatial order 208 -> 80, 70^3 FP64 344 -> 217,
+// 120^3 FP32 spatial 856 -> 634 (1.92 GB algorithmic: 3.0 TB/s), 120^3 FP64
+// 1294 -> 1046 (3.56 GB: 3.4 TB/s).
+template <typename T, int G, int P, int MINB>
+__global__ void __launch_bounds__(128, MINB)
+    k_trsv_flow(FlowSweep lo, FlowSweep up, const double *__restrict__ b, double *buf, size_t n, double *xout,
+                unsigned *ctl, int *err, uint32_t stage_blk)
+{
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t mbars[4][2];
+  constexpr int S = G / 4;   // quads per row: quad jj takes columns jj, jj + S, ...
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane & 3;
+  const int base = lane & ~(G - 1), jj = (lane & (G - 1)) >> 2;
+  const uint32_t W = gridDim.x * 4, total = lo.nc + up.nc;
+  const uint32_t stage_bytes = stage_blk * (16u * (uint32_t)sizeof(T) + 4u) + 32u;
+  unsigned char *stage0 = smem + (size_t)warp * 2 * stage_bytes;
+  const unsigned sel = *(volatile unsigned *)ctl & 1u;
+  double *y = buf, *x = buf + (1 + sel) * n, *xnext = buf + (2 - sel) * n;
+  if (lane == 0) {
+    mbar_init(&mbars[warp][0], 1);
+    mbar_init(&mbars[warp][1], 1);
+  }
+  __syncwarp();
+  auto desc = [&](uint32_t c) -> uint4 {
+    if (c >= total) return make_uint4(0, 0, 0, 0);
+    return c < lo.nc ? __ldg(lo.chunk + c) : __ldg(up.chunk + (c - lo.nc));
+  };
+  // a chunk's copies (lane 0) and its slots
+  auto issue = [&](uint32_t c, const uint4 &ch, int st) {
+    if (c >= total || lane != 0) return;
+    const FlowSweep &s = c < lo.nc ? lo : up;
+    unsigned char *dst = stage0 + (size_t)st * stage_bytes;
+    const uint32_t bb = (ch.w - ch.z) * 16u * (uint32_t)sizeof(T);
+    const uint32_t ca = ch.z & ~3u, cb = (((ch.w + 3u) & ~3u) - ca) * 4u;
+    mbar_expect_tx(&mbars[warp][st], bb + cb);
+    if (bb) bulk_g2s(dst, reinterpret_cast<const T *>(s.pk) + 16 * (size_t)ch.z, bb, &mbars[warp][st]);
+    if (cb) bulk_g2s(dst + (size_t)stage_blk * 16 * sizeof(T), s.col + ca, cb, &mbars[warp][st]);
+  };
+  auto slot_of = [&](uint32_t c, const uint4 &ch) -> uint4 {
+    const uint32_t s = ch.x + (uint32_t)(lane / G);
+    if (s >= ch.y) return make_uint4(0, 0, 0, 0xffffffffu);
+    return c < lo.nc ? __ldg(lo.slot + s) : __ldg(up.slot + s);
+  };
+  uint32_t c = warp * gridDim.x + blockIdx.x;   // consecutive chunks on different SMs
+  uint4 d0 = desc(c), d1 = desc(c + W);
+  issue(c, d0, 0);
+  issue(c + W, d1, 1);
+  uint4 s0 = slot_of(c, d0), s1 = slot_of(c + W, d1);
+  uint32_t phase = 0;
+  int st = 0;
+  bool failed = false;
+  for (; c < total; c += W) {
+    const uint4 dn = desc(c + 2 * W);
+    const bool upper = c >= lo.nc, active = s0.w != 0xffffffffu;
+    const size_t own = 4 * (size_t)s0.x + r;
+    double xi = 0.0;
+    if (active && !upper) xi = b[4 * (size_t)s0.w + r];
+    if (!__all_sync(0xffffffffu, mbar_wait(&mbars[warp][st], phase, err))) break;
+    const unsigned char *sg = stage0 + (size_t)st * stage_bytes;
+    const T *sa = reinterpret_cast<const T *>(sg) + 4 * r;
+    const uint32_t *sc = reinterpret_cast<const uint32_t *>(sg + (size_t)stage_blk * 16 * sizeof(T)) + (d0.z & 3u);
+    uint32_t k = active ? s0.y - d0.z : 0u, spins = 0;
+    const uint32_t ke = active ? s0.z - d0.z : 0u, kd = k;
+    // one more poll; after KF_SPIN_LIMIT of them, or when another wait gave
+    // up, no value is waited for any more
+    auto again = [&]() {
+      if (++spins > KF_SPIN_LIMIT) {
+        atomicExch(err, 1);
+        failed = true;
+      }
+      if ((spins & 255) == 0 && *(volatile int *)err) failed = true;
+      failed = __any_sync(0xffffffffu, failed);
+    };
+    if (upper && active) k++;   // the diagonal block comes first in the run
+    bool ywait = upper && active;
+    // the row's columns, S P at a time: all their values are asked for at
+    // once, and what is still missing is asked for again until the whole
+    // warp's are there; the products then run without branches (past a row's
+    // end they read whatever the stage holds and are not used)
+    const double *src = upper ? x : y;
+    do {
+      const uint32_t cnt = k < ke ? min(ke - k, (uint32_t)(S * P)) : 0u;
+      uint32_t pend = 0;
+      uint32_t col[P];
+      double4 v[P];
+#pragma unroll
+      for (int p = 0; p < P; p++) {
+        col[p] = sc[k + S * p + jj];
+        v[p] = make_double4(0.0, 0.0, 0.0, 0.0);
+        pend |= (uint32_t)((uint32_t)(S * p + jj) < cnt) << p;
+      }
+      while (true) {
+#pragma unroll
+        for (int p = 0; p < P; p++) ld_flow(v[p], src + 4 * (size_t)col[p], pend >> p & 1u);
+        if (ywait) {
+          xi = ld_flow1(y + own);
+          ywait = __double2hiint(xi) == -1;
+        }
+#pragma unroll
+        for (int p = 0; p < P; p++) pend &= ~((uint32_t)flow_ready(v[p]) << p);
+        if (failed) {
+          pend = 0u;
+          ywait = false;
+        }
+        if (!__any_sync(0xffffffffu, pend != 0u || ywait)) break;
+        again();
+      }
+      double t[P];
+#pragma unroll
+      for (int p = 0; p < P; p++) {
+        double a0, a1, a2, a3;
+        block_row(sa + 16 * (size_t)(k + S * p + jj), a0, a1, a2, a3);
+        double sum = 0.0;
+        sum += a0 * v[p].x;
+        sum += a1 * v[p].y;
+        sum += a2 * v[p].z;
+        sum += a3 * v[p].w;
+        t[p] = sum;
+      }
+#pragma unroll
+      for (int p = 0; p < P; p++)
+#pragma unroll
+        for (int j = 0; j < S; j++) {
+          const double u = S == 1 ? t[p] : __shfl_sync(0xffffffffu, t[p], base + 4 * j + r);
+          const double xn = -1.0 * u + xi;
+          xi = (uint32_t)(S * p + j) < cnt ? xn : xi;
+        }
+      k += cnt;
+    } while (__any_sync(0xffffffffu, k < ke));
+    if (!upper) {
+      if (active && jj == 0) {
+        st_flow(y + own, xi);
+        xnext[own] = __longlong_as_double(KF_FLOW_EMPTY);
+      }
+    } else {
+      const double x0 = __shfl_sync(0xffffffffu, xi, base + 0), x1 = __shfl_sync(0xffffffffu, xi, base + 1);
+      const double x2 = __shfl_sync(0xffffffffu, xi, base + 2), x3 = __shfl_sync(0xffffffffu, xi, base + 3);
+      if (active && jj == 0) {
+        double a0, a1, a2, a3;
+        block_row(sa + 16 * (size_t)kd, a0, a1, a2, a3);
+        double z = 0.0;
+        z += a0 * x0;
+        z += a1 * x1;
+        z += a2 * x2;
+        z += a3 * x3;
+        st_flow(x + own, z);
+        xout[4 * (size_t)s0.w + r] = z;
+        y[own] = __longlong_as_double(KF_FLOW_EMPTY);
+      }
+    }
+    __syncwarp();   // every lane is done with the stage
+    issue(c + 2 * W, dn, st);
+    d0 = d1;
+    s0 = s1;
+    d1 = dn;
+    s1 = slot_of(c + 2 * W, dn);
+    st ^= 1;
+    if (st == 0) phase ^= 1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(ctl + 1, 1u) == gridDim.x - 1) {
+    ctl[1] = 0;
+    ctl[0] = sel ^ 1u;
+  }
+}
+
 // ------------------------------------------------------------------ J.v
 
 // src/kernel.c:35-44: y = (y - r + cdt (w - q)) * a, a = |x| / h from the
@@ -2275,6 +2517,14 @@ void fill(DevMesh &m, const double *q, double u, double v, int precision)
 
 static void packed_setup();
 
+// The data-flow sweeps serve the active pattern: mode 8, and no row longer
+// than their shared-memory stage.
+static bool flow_fits(const DevMesh &m)
+{
+  return m.pk_flow && m.trsv_mode == 8 && m.pk[0].chunk[2] && m.pk[1].chunk[2] &&
+         std::max(m.pk[0].maxblk[2], m.pk[1].maxblk[2]) <= KF_FLOW_ROW_MAX;
+}
+
 void ilu(DevMesh &m, int precision)
 {
   int *status = m.status;
@@ -2308,7 +2558,7 @@ void ilu(DevMesh &m, int precision)
   else
     k_ilu_finish_f32<<<blocks((size_t)m.N * 16, 256), 256, 0, m.stream>>>(m.N, m.diag, m.dinvf, m.Af);
   kf_count_launch();
-  if (m.trsv_mode == 8 && m.pk[0].chunk[0] && (precision == 1 || m.pk_fp64)) {
+  if (m.trsv_mode == 8 && m.pk[0].chunk[0] && (precision == 1 || m.pk_fp64 || flow_fits(m))) {
     packed_setup();
     for (int pass = 0; pass < 2; pass++) {
       const uint32_t nb = m.pk[pass].nblk, off = pass == 0 ? 0u : m.pk[0].nblk;
@@ -2403,11 +2653,60 @@ static void sptrsv_packed(DevMesh &m, const double *b, double *x, const uint32_t
   }
 }
 
+// Both sweeps through k_trsv_flow (flow_fits): one cooperative launch of as
+// many CTAs as are resident at once, or as the chunks fill.  b and x in the
+// mesh's numbering whatever the pattern's.
+template <typename T> static void sptrsv_flow(DevMesh &m, const double *b, double *x)
+{
+  const void *fn = m.flow_lanes == 8 ? (const void *)k_trsv_flow<T, 8, 4, sizeof(T) == 4 ? 5 : 4>
+                                       : (const void *)k_trsv_flow<T, 4, 8, sizeof(T) == 4 ? 4 : 3>;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  const T *P = reinterpret_cast<const T *>(m.pk_buf);
+  FlowSweep s[2];
+  for (int i = 0; i < 2; i++)
+    s[i] = FlowSweep{m.pk[i].chunk[2], m.pk[i].slot, m.pk[i].col, P + (i ? 16 * (size_t)m.pk[0].nblk : (size_t)0),
+                     m.pk[i].lev[2].back()};
+  uint32_t stage = (std::max(m.pk[0].maxblk[2], m.pk[1].maxblk[2]) + 3u) & ~3u;   // 16-byte aligned stages
+  // (the 16 blocks after the last stage may be read past a row's end, unused)
+  const size_t smem = 8 * ((size_t)stage * (16 * sizeof(T) + 4) + 32) + 16 * 16 * sizeof(T);
+  int per = 0, nsm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 128, smem);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m.device);
+  const uint32_t nc = s[0].nc + s[1].nc;
+  size_t n = 4 * (size_t)m.N;
+  int *err = m.status + 1;
+  void *args[] = {&s[0], &s[1], (void *)&b, (void *)&m.flow_buf, &n, (void *)&x, (void *)&m.flow_ctl, (void *)&err,
+                  &stage};
+  cudaLaunchConfig_t cfg = {};
+  // three levels' chunks at most: a warp whose rows are many levels ahead only
+  // loads the memory system with its polls (25^3, FP64: 92 us with every
+  // resident warp, 83 us with three levels' worth, 90 and 135 us with two and
+  // one)
+  const uint32_t ahead = (uint32_t)(3.0 * nc / (double)(m.nlev_l + m.nlev_u) / 4.0) + 1;
+  cfg.gridDim = dim3(std::min(std::min((uint32_t)(std::max(per, 1) * nsm), ahead), std::max(1u, (nc + 3) / 4)));
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = m.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+  if (e != cudaSuccess) kf_set_error(KFUN3D_ERR_CUDA, cudaGetErrorString(e));
+  kf_count_launch();
+}
+
 // x = P^T (LU)^-1 P b for a renumbered pattern (m.row_node) through the
 // packed schedule, the permutations folded into its first and last sweeps;
 // false (nothing done) when the active schedule is not the packed one.
 bool sptrsv_permuted(DevMesh &m, const double *b, double *x, int precision)
 {
+  if (m.row_node && flow_fits(m)) {
+    if (precision == 0) sptrsv_flow<double>(m, b, x);
+    else sptrsv_flow<float>(m, b, x);
+    return true;
+  }
   const int mode = (m.trsv_mode == 8 && precision == 0 && !m.pk_fp64) ? 7 : m.trsv_mode;
   if (mode != 8 || !m.pk[0].chunk[0] || !m.row_node) return false;
   if (precision == 0) sptrsv_packed<double>(m, b, m.px, m.row_node, x);
@@ -2447,8 +2746,16 @@ int bounded_wait_check(cudaStream_t st)
 
 void sptrsv(DevMesh &m, const double *b, double *x, int precision)
 {
-  // the packed schedule serves FP32 factors; FP64 factors take the four-lane
-  // level launches unless m.pk_fp64 (measured faster at 120^3 in both orders)
+  // (the other schedules run in the pattern's own numbering: a renumbered
+  // pattern's data-flow sweeps are sptrsv_permuted's)
+  if (!m.row_node && flow_fits(m)) {
+    if (precision == 0) sptrsv_flow<double>(m, b, x);
+    else sptrsv_flow<float>(m, b, x);
+    return;
+  }
+  // the packed level launches serve FP32 factors; FP64 factors take the
+  // four-lane level launches unless m.pk_fp64 (measured faster at 120^3 in
+  // both orders)
   const int mode = (m.trsv_mode == 8 && precision == 0 && !m.pk_fp64) ? 7 : m.trsv_mode;
   if (mode == 8 && m.pk[0].chunk[0]) {
     if (precision == 0) sptrsv_packed<double>(m, b, x);
@@ -2614,6 +2921,11 @@ void sptrsv(DevMesh &m, const double *b, double *x, int precision)
 // here), for the allocation-free entry point in noalloc.cu.
 void sptrsv_flags(DevMesh &m, const double *b, double *x, int precision, uint32_t *flags)
 {
+  if (!m.row_node && flow_fits(m)) {
+    if (precision == 0) sptrsv_flow<double>(m, b, x);
+    else sptrsv_flow<float>(m, b, x);
+    return;
+  }
   cudaMemsetAsync(flags, 0, (size_t)m.N * sizeof(uint32_t), m.stream);
   const double *bb = b;
   uint32_t N = m.N, eL = 1, eU = 2;

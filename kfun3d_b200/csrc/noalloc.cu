@@ -126,6 +126,7 @@ extern "C" int kfun3d_sptrsv_device_noalloc(const GEOMETRY *g, const double *d_b
   e = cudaMemcpy(st, m.status, sizeof(st), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && st[1]) {
     cudaMemset(m.status + 1, 0, sizeof(int));
+    kf_flow_reset(m);
     kf_set_error(KFUN3D_ERR_TIMEOUT, "kfun3d_sptrsv_device_noalloc: a triangular-solve wait exceeded its bound");
     return KFUN3D_ERR_TIMEOUT;
   }

@@ -433,13 +433,15 @@ __global__ void k_visit_nodes(uint32_t N, const uint32_t *__restrict__ ord, cons
 // row's blocks of its descriptor's range, in column order
 __global__ void k_packed_streams(uint32_t N, bool upper, const uint4 *__restrict__ desc,
                                  const uint32_t *__restrict__ first, const uint32_t *__restrict__ ja,
-                                 const uint32_t *__restrict__ diag, uint32_t *row, uint32_t *col, uint32_t *src)
+                                 const uint32_t *__restrict__ diag, const uint32_t *__restrict__ row_node,
+                                 uint32_t *row, uint32_t *col, uint32_t *src, uint4 *slot)
 {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= N) return;
   const uint4 d = desc[q];
   uint32_t k = first[q];
   row[q] = d.x;
+  slot[q] = make_uint4(d.x, k, first[q + 1], row_node ? row_node[d.x] : d.x);
   if (upper) {
     col[k] = d.x;
     src[k++] = diag[d.x];
@@ -818,10 +820,11 @@ int kf_build_mesh_lists_device(DevMesh &m, const GEOMETRY *g)
 }
 
 int kf_packed_streams_device(uint32_t N, bool upper, const uint4 *desc, const uint32_t *first, const uint32_t *ja,
-                             const uint32_t *diag, uint32_t *row, uint32_t *col, uint32_t *src, cudaStream_t st)
+                             const uint32_t *diag, const uint32_t *row_node, uint32_t *row, uint32_t *col,
+                             uint32_t *src, uint4 *slot, cudaStream_t st)
 {
   if (N) {
-    k_packed_streams<<<nblk(N, 256), 256, 0, st>>>(N, upper, desc, first, ja, diag, row, col, src);
+    k_packed_streams<<<nblk(N, 256), 256, 0, st>>>(N, upper, desc, first, ja, diag, row_node, row, col, src, slot);
     kf_count_launch();
   }
   return cudaGetLastError() == cudaSuccess ? KFUN3D_OK : KFUN3D_ERR_CUDA;

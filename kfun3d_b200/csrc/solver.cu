@@ -794,6 +794,7 @@ int device_status(DevMesh &m)
     CK(cudaMemsetAsync(m.status, 0, 2 * sizeof(int), m.stream));
     // a wait that gave up may leave a grid barrier half-counted
     if (st[1] && m.bar) CK(cudaMemsetAsync(m.bar, 0, 8 * sizeof(unsigned), m.stream));
+    if (st[1] && m.flow_buf) CK(kf_flow_reset(m));
   }
   if (st[1]) return KFUN3D_ERR_TIMEOUT;
   return st[0];
