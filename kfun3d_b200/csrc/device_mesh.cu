@@ -440,7 +440,7 @@ static void release_device(MatrixHandle *h)
                   m->wf_n, m->s_n, m->f_n, m->bnd_of, m->bnd_node, m->bnd_ptr, m->bnd_ent, m->ia, m->ja,
                   m->diag, m->tblk, m->lpos, m->last_lower, m->lev_l, m->lev_u, m->A, m->lslot, m->dinv,
                   m->Af, m->dinvf, m->q, m->r, m->gx, m->gy, m->gz, m->cdt, m->w, m->t, m->x, m->rhs, m->V,
-                  m->red, m->scal, m->forces, m->dscr, m->status, m->flags, m->ticket, m->part, m->lsq_coef,
+                  m->red, m->scal, m->forces, m->dscr, m->status, m->flags, m->ticket, m->gs_part, m->lsq_coef,
                   m->qv, m->xyzv, m->gxv, m->gyv, m->gzv, m->inc_othv, m->n0v, m->n1v, m->inc_geo, m->desc_l, m->desc_u, m->eoff, m->n1, m->in1_ptr, m->in1_edge, m->eres, m->n0s, m->pair_ptr, m->pairs, m->lev_ptr_d, m->bar, m->Z, m->qold, m->fy, m->fx, m->pscr, m->ord, m->rowof, m->egeo_s, m->sub_part};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -584,7 +584,7 @@ extern "C" long kfun3d_device_query(const GEOMETRY *g, const char *key)
   if (strcmp(key, "sptrsv_schedule") == 0) return m->trsv_mode;
   if (strcmp(key, "lsq_terms_match") == 0) return m->lsq_match ? 1 : 0;
   if (strcmp(key, "visit_order_copies") == 0) return m->visit ? 1 : 0;
-  if (strcmp(key, "mgs_resident") == 0) return m->mgs_resident ? 1 : 0;
+  if (strcmp(key, "mgs_resident") == 0) return 0;   // (no Gram-Schmidt kernel keeps the vector on chip any more)
   if (strcmp(key, "setup_us") == 0) return m->setup_us;
   if (strcmp(key, "pattern_us") == 0) return m->pattern_us;
   if (strcmp(key, "spatial_setup_us") == 0) return m->spatial_us;
@@ -863,6 +863,8 @@ DevMesh *kf_device(const GEOMETRY *g)
   KF_CUDA(cudaMalloc(&m->red, 4096 * sizeof(double)));
   KF_CUDA(cudaMalloc(&m->scal, 256 * sizeof(double)));
   KF_CUDA(cudaMemset(m->scal, 0, 256 * sizeof(double)));
+  KF_CUDA(cudaMalloc(&m->gs_part, (64 * 296 + 32 * 32) * sizeof(double)));
+  KF_CUDA(cudaMemset(m->gs_part, 0, (64 * 296 + 32 * 32) * sizeof(double)));
   KF_CUDA(cudaMalloc(&m->forces, 4 * sizeof(double)));
   KF_CUDA(cudaMalloc(&m->status, 4 * sizeof(int)));
   KF_CUDA(cudaMemset(m->status, 0, 4 * sizeof(int)));

@@ -357,12 +357,9 @@ struct DevMesh {
   unsigned arnoldi_nodes[2][2][KF_NBASIS] = {};
   double graph_aoa = 0.0;
   bool use_graphs = true;
-  unsigned mgs_grid = 0;          // cooperative grid for the Gram-Schmidt kernel
-  bool mgs_resident = true;       // Gram-Schmidt with w kept on chip (k_mgs_resident)
-  int mgs_ts = 0;                 // its double2 elements per thread in shared memory
-  double *part = nullptr;         // [2][mgs_grid] block partial sums
-  unsigned *bar = nullptr;        // grid-barrier words: [0..1] persistent sweep, [2..3] Gram-Schmidt,
-                                  // [4] counter of the one-CTA-per-SM sweep
+  double *gs_part = nullptr;      // [64][296] block partial sums, [32][32] lower triangle of the basis' Gram matrix
+  unsigned *bar = nullptr;        // grid-barrier words: [0..1] persistent sweep, arrivals of [2..3]
+                                  // Gram-Schmidt; [4] counter of the one-CTA-per-SM sweep
   uint32_t *lev_ptr_d = nullptr;  // [nlev_l+1 + nlev_u+1] level offsets on the device
   unsigned trsv_pgrid = 0;        // persistent sweep grid
   unsigned trsv_mgrid = 0;        // persistent sweep grid of mode 5 (SMs x trsv_mgrid_per)

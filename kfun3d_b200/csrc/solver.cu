@@ -133,13 +133,6 @@ __global__ void k_dot_final(const double *__restrict__ part, int np, double *__r
   }
 }
 
-// Fast-mode modified Gram-Schmidt of V[k+1] against V[0..k] and its
-// normalisation (src/kernel.c:129-141) in one cooperative launch.  Pass v
-// applies the previous projection, w -= h[v-1] V[v-1], and forms the block
-// partial sums of w.V[v] in the same sweep; after a grid-wide barrier every
-// block adds the partial sums in the same fixed order, so all blocks hold the
-// identical h[v] (run-to-run deterministic).  Partial sums alternate between
-// two buffers, so one barrier per projection suffices.
 __device__ __forceinline__ double block_sum(double v, double *sm)
 {
   v = warp_sum(v);
@@ -167,224 +160,166 @@ __device__ __forceinline__ double grid_total(const double *part, int np, double 
   return t;
 }
 
-constexpr int KF_MGS_ELEMS = 8;   // double2 elements per thread kept in registers
+// Fast-mode modified Gram-Schmidt of w = V[k+1] against V[0..k] and its
+// normalisation (src/kernel.c:129-141) with two reductions instead of k + 2:
+// the coefficients h_v = V_v . (w - sum_{j<v} h_j V_j) of the sequential sweep
+// are h_v = V_v . w - sum_{j<v} h_j (V_v . V_j), so all the products V_v . w are
+// formed in one pass (k_gs_dots), with those of V_k against V_0..V_{k-1}, which
+// complete the strictly lower triangle L of the basis' Gram matrix (one row a
+// step); (I + L) h = V^T w is solved by substitution, and w -= V h takes one
+// more pass (k_gs_update).  The basis is not assumed orthonormal, as in the
+// sequential sweep.  Every sum has a fixed shape: run-to-run deterministic.
+//
+// Bound by memory on large meshes (the basis is read twice, once in groups of
+// GS_GROUP with w and V_k read again per group: (k+1)(2 + 2/8) + 4 vectors) and
+// by three launches on small ones, where the sequential sweep paid a grid
+// barrier of about 6 us per projection.  At Arnoldi index 15, sweep with the
+// vector kept on chip / now: 25^3 102 / 21 us, 40^3 107 / 27, 70^3 138 / 72,
+// 120^3 426 / 342 us (2.2 GB, 6.4 TB/s).
+constexpr int GS_BLOCKS = 296;   // 2 x 148 SMs
+constexpr int GS_GROUP = 8;      // basis vectors a pass over w takes at once
 
-__global__ void __launch_bounds__(256, 3) k_mgs_coop(size_t n, double *__restrict__ V, int k,
-                                                     double *__restrict__ h, double *__restrict__ part,
-                                                     unsigned *bar, int *err)
+// The last CTA of a grid to arrive (its partial sums written before): true in
+// every thread of that CTA, which then sees all partial sums.  Resets *cnt.
+__device__ __forceinline__ bool last_cta(unsigned *cnt)
 {
-  __shared__ double sm[40];
-  const int G = gridDim.x;
-  const size_t n2 = n / 2;
-  double2 *w = reinterpret_cast<double2 *>(V + (size_t)(k + 1) * n);
-  const size_t stride = (size_t)G * blockDim.x;
+  __shared__ bool last_s;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last_s = atomicAdd(cnt, 1u) == gridDim.x - 1;
+    if (last_s) *cnt = 0;
+  }
+  __syncthreads();
+  if (last_s) __threadfence();
+  return last_s;
+}
+
+// part: [2 (k + 1)][GS_BLOCKS] partial sums (w, then V_k, against each vector);
+// L: [KF_NBASIS][32], row v = V_v . V_j for j < v
+__global__ void __launch_bounds__(256, 2) k_gs_dots(size_t n, const double *__restrict__ V, int k,
+                                                    double *__restrict__ h, double *__restrict__ part,
+                                                    double *__restrict__ L, unsigned *cnt)
+{
+  __shared__ double sm[8][2 * GS_GROUP];
+  __shared__ double tot[2 * 32];
+  const size_t n2 = n / 2, stride = (size_t)gridDim.x * blockDim.x;
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t iend_reg = i0 + KF_MGS_ELEMS * stride;   // elements beyond are re-read from memory
-  double2 pv[KF_MGS_ELEMS];   // this thread's elements of the previous basis vector
-  double hprev = 0.0;
-  for (int v = 0; v <= k + 1; v++) {
-    const double2 *prev = v > 0 ? reinterpret_cast<const double2 *>(V + (size_t)(v - 1) * n) : nullptr;
-    const double2 *cur = v <= k ? reinterpret_cast<const double2 *>(V + (size_t)v * n) : nullptr;
-    double s = 0.0;
+  const double2 *w = reinterpret_cast<const double2 *>(V + (size_t)(k + 1) * n);
+  const double2 *vk = reinterpret_cast<const double2 *>(V + (size_t)k * n);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int g0 = 0; g0 <= k; g0 += GS_GROUP) {
+    double s[2 * GS_GROUP];
 #pragma unroll
-    for (int t = 0; t < KF_MGS_ELEMS; t++) {
-      const size_t i = i0 + (size_t)t * stride;
-      if (i < n2) {
-        double2 a = w[i];
-        if (v > 0) {
-          a.x = fma(-hprev, pv[t].x, a.x);
-          a.y = fma(-hprev, pv[t].y, a.y);
-          w[i] = a;
-        }
-        if (cur) {
-          const double2 c = __ldcs(cur + i);
-          s = fma(a.x, c.x, s);
-          s = fma(a.y, c.y, s);
-          pv[t] = c;
-        } else {
-          s = fma(a.x, a.x, s);
-          s = fma(a.y, a.y, s);
-        }
+    for (int u = 0; u < 2 * GS_GROUP; u++) s[u] = 0.0;
+    for (size_t i = i0; i < n2; i += stride) {
+      const double2 a = w[i], b = vk[i];
+      double2 c[GS_GROUP];
+#pragma unroll
+      for (int u = 0; u < GS_GROUP; u++) {
+        c[u] = b;   // V_k itself (and a filler beyond it)
+        if (g0 + u < k) c[u] = __ldcs(reinterpret_cast<const double2 *>(V + (size_t)(g0 + u) * n) + i);
+      }
+#pragma unroll
+      for (int u = 0; u < GS_GROUP; u++) {
+        s[u] = fma(a.x, c[u].x, s[u]);
+        s[u] = fma(a.y, c[u].y, s[u]);
+        s[GS_GROUP + u] = fma(b.x, c[u].x, s[GS_GROUP + u]);
+        s[GS_GROUP + u] = fma(b.y, c[u].y, s[GS_GROUP + u]);
       }
     }
-    for (size_t i = iend_reg; i < n2; i += stride) {
-      double2 a = w[i];
-      if (prev) {
-        const double2 p = prev[i];
-        a.x = fma(-hprev, p.x, a.x);
-        a.y = fma(-hprev, p.y, a.y);
-        w[i] = a;
-      }
-      if (cur) {
-        const double2 c = cur[i];
-        s = fma(a.x, c.x, s);
-        s = fma(a.y, c.y, s);
-      } else {
-        s = fma(a.x, a.x, s);
-        s = fma(a.y, a.y, s);
+#pragma unroll
+    for (int u = 0; u < 2 * GS_GROUP; u++) {
+      const double v = warp_sum(s[u]);
+      if (lane == 0) sm[warp][u] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 * GS_GROUP) {
+      const int u = threadIdx.x % GS_GROUP, which = threadIdx.x / GS_GROUP;
+      if (g0 + u <= k) {
+        double v = 0.0;
+        for (int x = 0; x < 8; x++) v += sm[x][threadIdx.x];
+        part[(size_t)(2 * (g0 + u) + which) * GS_BLOCKS + blockIdx.x] = v;
       }
     }
-    double *pb = part + (v & 1) * G;
-    const double bs = block_sum(s, sm);
-    if (threadIdx.x == 0) pb[blockIdx.x] = bs;
-    __threadfence();
-    if (!kf_grid_barrier(bar, err)) return;
-    const double tot = grid_total(pb, G, sm);
-    if (v <= k) {
-      hprev = tot;
-      if (blockIdx.x == 0 && threadIdx.x == 0) h[v] = tot;
-    } else {
-      const double nrm = sqrt(tot);
-      if (blockIdx.x == 0 && threadIdx.x == 0) h[k + 1] = nrm;
-      const double sc = 1.0 / nrm;
-      for (size_t i = i0; i < n2; i += stride) {
-        double2 a = w[i];
-        a.x *= sc;
-        a.y *= sc;
-        w[i] = a;
-      }
+    __syncthreads();
+  }
+  if (!last_cta(cnt)) return;
+  for (int q = warp; q < 2 * (k + 1); q += 8) {
+    double v = 0.0;
+    for (int x = lane; x < (int)gridDim.x; x += 32) v += __ldcg(part + (size_t)q * GS_BLOCKS + x);
+    v = warp_sum(v);
+    if (lane == 0) tot[q] = v;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // forward substitution, lane v = coefficient v
+    if (lane < k) L[32 * k + lane] = tot[2 * lane + 1];
+    double hv = lane <= k ? tot[2 * lane] : 0.0;
+    for (int j = 0; j < k; j++) {
+      const double hj = __shfl_sync(0xffffffffu, hv, j);
+      const double l = lane > j && lane <= k ? (lane == k ? tot[2 * j + 1] : L[32 * lane + j]) : 0.0;
+      if (lane > j) hv = fma(-l, hj, hv);
     }
+    if (lane <= k) h[lane] = hv;
   }
 }
 
-// The same modified Gram-Schmidt with the vector being orthogonalised, w,
-// resident on chip for the whole launch: each thread keeps its first
-// KF_MGS_REG double2 elements of w in registers and the next `ts` in shared
-// memory (the rest, on meshes too large for that, stays in global memory).
-// A sweep then reads only the previous basis vector (just read by the sweep
-// before, so mostly an L2 hit) and the current one from memory, instead of
-// reading and writing w as well.  One CTA of 512 threads per SM; element i of
-// thread g (grid-wide) is g + t * stride for t = 0, 1, ...  The arithmetic is
-// k_mgs_coop's: per thread the same fma chain in the same element order,
-// block sums and the fixed-order grid total unchanged in form.
-constexpr int KF_MGS_REG = 16;    // double2 elements per thread in registers
-constexpr int KF_MGS_BATCH = 4;   // elements whose loads are in flight together
-
-__global__ void __launch_bounds__(512, 1) k_mgs_resident(size_t n, double *__restrict__ V, int k,
-                                                         double *__restrict__ h, double *__restrict__ part,
-                                                         unsigned *bar, int *err, int ts)
+// w -= sum_v h[v] V[v] (in that order) and h[k+1] = |w|.  Elements from the
+// last to the first: those k_gs_dots read last may still be in L2.
+__global__ void __launch_bounds__(256, 3) k_gs_update(size_t n, double *__restrict__ V, int k,
+                                                      double *__restrict__ h, double *__restrict__ part,
+                                                      unsigned *cnt)
 {
-  extern __shared__ double2 wsm[];   // [ts][blockDim.x]
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ double sm[40];
-  const int G = gridDim.x;
-  const size_t n2 = n / 2;
-  double2 *w = reinterpret_cast<double2 *>(V + (size_t)(k + 1) * n);
-  const size_t stride = (size_t)G * blockDim.x;
+  __shared__ double hs[32];
+  if (threadIdx.x <= k) hs[threadIdx.x] = h[threadIdx.x];
+  __syncthreads();
+  const size_t n2 = n / 2, stride = (size_t)gridDim.x * blockDim.x;
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t tcache = (size_t)KF_MGS_REG + (size_t)ts;   // elements t below this are on chip
-  double2 wr[KF_MGS_REG];
+  double2 *w = reinterpret_cast<double2 *>(V + (size_t)(k + 1) * n);
+  double s = 0.0;
+  for (size_t j = i0; j < n2; j += stride) {
+    const size_t i = n2 - 1 - j;
+    double2 a = w[i];
+    int v = 0;
+    for (; v + 8 <= k + 1; v += 8) {
+      double2 c[8];
 #pragma unroll
-  for (int t = 0; t < KF_MGS_REG; t++) {
-    const size_t i = i0 + (size_t)t * stride;
-    wr[t] = i < n2 ? w[i] : make_double2(0.0, 0.0);
+      for (int u = 0; u < 8; u++) c[u] = reinterpret_cast<const double2 *>(V + (size_t)(v + u) * n)[i];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        a.x = fma(-hs[v + u], c[u].x, a.x);
+        a.y = fma(-hs[v + u], c[u].y, a.y);
+      }
+    }
+    for (; v <= k; v++) {
+      const double2 c = reinterpret_cast<const double2 *>(V + (size_t)v * n)[i];
+      a.x = fma(-hs[v], c.x, a.x);
+      a.y = fma(-hs[v], c.y, a.y);
+    }
+    w[i] = a;
+    s = fma(a.x, a.x, s);
+    s = fma(a.y, a.y, s);
   }
-  for (int t = 0; t < ts; t++) {
-    const size_t i = i0 + (size_t)(KF_MGS_REG + t) * stride;
-    wsm[(size_t)t * blockDim.x + threadIdx.x] = i < n2 ? w[i] : make_double2(0.0, 0.0);
-  }
-  double hprev = 0.0;
-  for (int v = 0; v <= k + 1; v++) {
-    const double2 *prev = v > 0 ? reinterpret_cast<const double2 *>(V + (size_t)(v - 1) * n) : nullptr;
-    const double2 *cur = v <= k ? reinterpret_cast<const double2 *>(V + (size_t)v * n) : nullptr;
-    double s = 0.0;
-    // elements in batches of KF_MGS_BATCH: all their loads are issued before
-    // any is used, so a thread keeps that many pairs of loads in flight
-    double2 pv[KF_MGS_BATCH], cv[KF_MGS_BATCH];
-    auto load = [&](int u, size_t i) {
-      if (prev) pv[u] = prev[i];
-      if (cur) cv[u] = cur[i];
-    };
-    auto step = [&](double2 &a, int u) {
-      if (prev) {
-        a.x = fma(-hprev, pv[u].x, a.x);
-        a.y = fma(-hprev, pv[u].y, a.y);
-      }
-      if (cur) {
-        s = fma(a.x, cv[u].x, s);
-        s = fma(a.y, cv[u].y, s);
-      } else {
-        s = fma(a.x, a.x, s);
-        s = fma(a.y, a.y, s);
-      }
-    };
-#pragma unroll
-    for (int t0 = 0; t0 < KF_MGS_REG; t0 += KF_MGS_BATCH) {
-#pragma unroll
-      for (int u = 0; u < KF_MGS_BATCH; u++) {
-        const size_t i = i0 + (size_t)(t0 + u) * stride;
-        if (i < n2) load(u, i);
-      }
-#pragma unroll
-      for (int u = 0; u < KF_MGS_BATCH; u++) {
-        const size_t i = i0 + (size_t)(t0 + u) * stride;
-        if (i < n2) step(wr[t0 + u], u);
-      }
-    }
-    for (int t0 = 0; t0 < ts; t0 += KF_MGS_BATCH) {
-#pragma unroll
-      for (int u = 0; u < KF_MGS_BATCH; u++) {
-        const size_t i = i0 + (size_t)(KF_MGS_REG + t0 + u) * stride;
-        if (t0 + u < ts && i < n2) load(u, i);
-      }
-#pragma unroll
-      for (int u = 0; u < KF_MGS_BATCH; u++) {
-        const size_t i = i0 + (size_t)(KF_MGS_REG + t0 + u) * stride;
-        if (t0 + u < ts && i < n2) {
-          double2 a = wsm[(size_t)(t0 + u) * blockDim.x + threadIdx.x];
-          step(a, u);
-          wsm[(size_t)(t0 + u) * blockDim.x + threadIdx.x] = a;
-        }
-      }
-    }
-    for (size_t i0g = i0 + tcache * stride; i0g < n2; i0g += KF_MGS_BATCH * stride) {
-#pragma unroll
-      for (int u = 0; u < KF_MGS_BATCH; u++) {
-        const size_t i = i0g + (size_t)u * stride;
-        if (i < n2) load(u, i);
-      }
-#pragma unroll
-      for (int u = 0; u < KF_MGS_BATCH; u++) {
-        const size_t i = i0g + (size_t)u * stride;
-        if (i < n2) {
-          double2 a = w[i];
-          step(a, u);
-          if (prev) w[i] = a;
-        }
-      }
-    }
-    double *pb = part + (v & 1) * G;
-    const double bs = block_sum(s, sm);
-    if (threadIdx.x == 0) pb[blockIdx.x] = bs;
-    __threadfence();
-    if (!kf_grid_barrier(bar, err)) return;
-    const double tot = grid_total(pb, G, sm);
-    if (v <= k) {
-      hprev = tot;
-      if (blockIdx.x == 0 && threadIdx.x == 0) h[v] = tot;
-    } else {
-      const double nrm = sqrt(tot);
-      if (blockIdx.x == 0 && threadIdx.x == 0) h[k + 1] = nrm;
-      const double sc = 1.0 / nrm;
-#pragma unroll
-      for (int t = 0; t < KF_MGS_REG; t++) {
-        const size_t i = i0 + (size_t)t * stride;
-        if (i < n2) w[i] = make_double2(wr[t].x * sc, wr[t].y * sc);
-      }
-      for (int t = 0; t < ts; t++) {
-        const size_t i = i0 + (size_t)(KF_MGS_REG + t) * stride;
-        if (i < n2) {
-          const double2 a = wsm[(size_t)t * blockDim.x + threadIdx.x];
-          w[i] = make_double2(a.x * sc, a.y * sc);
-        }
-      }
-      for (size_t i = i0 + tcache * stride; i < n2; i += stride) {
-        double2 a = w[i];
-        a.x *= sc;
-        a.y *= sc;
-        w[i] = a;
-      }
-    }
-  }
+  const double bs = block_sum(s, sm);
+  if (threadIdx.x == 0) part[blockIdx.x] = bs;
+  if (!last_cta(cnt)) return;
+  const double t = grid_total(part, gridDim.x, sm);
+  if (threadIdx.x == 0) h[k + 1] = sqrt(t);
+}
+
+// w /= |w|
+__global__ void __launch_bounds__(256) k_gs_scale(size_t n, double *__restrict__ V, int k, const double *__restrict__ h)
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n / 2) return;
+  double2 *w = reinterpret_cast<double2 *>(V + (size_t)(k + 1) * n);
+  const double sc = 1.0 / h[k + 1];
+  const double2 a = w[i];
+  w[i] = make_double2(a.x * sc, a.y * sc);
 }
 
 // y = (mult * coef[0]) * x + y with the coefficient on the device
@@ -692,53 +627,30 @@ void dev_normalize(DevMesh &m, double *x, double *nrm, bool fast)
   kf_count_launch();
 }
 
-// Gram-Schmidt kernel: k_mgs_resident (default, w kept on chip) or
-// k_mgs_coop (KFUN3D_MGS=coop); grid and shared memory fixed per mesh.
-void mgs_coop_prepare(DevMesh &m)
+template <class... P, class... A>
+void launch_dependent(void (*kern)(P...), unsigned grid, cudaStream_t st, A... args)
 {
-  if (!m.mgs_grid) {
-    int nsm = 0, per = 0, smax = 0;
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m.device));
-    const char *env = getenv("KFUN3D_MGS");
-    m.mgs_resident = !(env && strcmp(env, "coop") == 0);
-    if (m.mgs_resident) {
-      CK(cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, m.device));
-      const size_t n2 = 2 * (size_t)m.N, stride = (size_t)nsm * 512;
-      const size_t per_thread = (n2 + stride - 1) / stride;
-      const size_t room = (size_t)std::max(smax - 1024, 0) / (512 * sizeof(double2));
-      m.mgs_ts = (int)std::min(room, per_thread > (size_t)KF_MGS_REG ? per_thread - KF_MGS_REG : (size_t)0);
-      CK(cudaFuncSetAttribute((const void *)k_mgs_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(m.mgs_ts * 512 * sizeof(double2))));
-      m.mgs_grid = (unsigned)nsm;
-    } else {
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mgs_coop, 256, 0));
-      m.mgs_grid = (unsigned)nsm * (unsigned)std::min(std::max(per, 1), 3);
-    }
-    CK(cudaMalloc(&m.part, 2 * m.mgs_grid * sizeof(double)));
-  }
-}
-
-void mgs_coop(DevMesh &m, int k)
-{
-  mgs_coop_prepare(m);
-  size_t n = 4 * (size_t)m.N;
-  double *V = m.V, *h = m.scal, *part = m.part;
-  unsigned *bar = m.bar + 2;
-  int *err = m.status + 1;
-  int ts = m.mgs_ts;
-  void *args[] = {&n, &V, &k, &h, &part, &bar, &err, &ts};
+  // starts while the kernel before it ends (it waits for it with griddepcontrol.wait)
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(m.mgs_grid);
-  cfg.blockDim = dim3(m.mgs_resident ? 512 : 256);
-  cfg.dynamicSmemBytes = m.mgs_resident ? (size_t)m.mgs_ts * 512 * sizeof(double2) : 0;
-  cfg.stream = m.stream;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CK(cudaLaunchKernelExC(&cfg, m.mgs_resident ? (const void *)k_mgs_resident : (const void *)k_mgs_coop, args));
-  kf_count_launch();
+  CK(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+
+void gram_schmidt(DevMesh &m, int k)
+{
+  const size_t n = 4 * (size_t)m.N;
+  const unsigned grid = std::min((unsigned)GS_BLOCKS, std::max(1u, nblk(n / 2, 256)));
+  k_gs_dots<<<grid, 256, 0, m.stream>>>(n, m.V, k, m.scal, m.gs_part, m.gs_part + 64 * GS_BLOCKS, m.bar + 2);
+  launch_dependent(k_gs_update, grid, m.stream, n, m.V, k, m.scal, m.gs_part, m.bar + 3);
+  launch_dependent(k_gs_scale, std::max(1u, nblk(n / 2, 256)), m.stream, n, m.V, k, (const double *)m.scal);
+  kf_count_launch(3);
 }
 
 // One Arnoldi step k (src/kernel.c:123-141): V[k+1] = M^-1 J V[k],
@@ -748,7 +660,7 @@ void orthogonalize(DevMesh &m, const Ops &o, int k)
 {
   const size_t n = 4 * (size_t)m.N;
   if (o.fast && (n % 2) == 0) {
-    mgs_coop(m, k);
+    gram_schmidt(m, k);
     return;
   }
   for (int v = 0; v <= k; v++) {
@@ -765,7 +677,7 @@ void arnoldi_step(DevMesh &m, const Ops &o, int k, int prec)
   dev_jacvec(m, o, Vb(m, k), m.t);
   o.sptrsv(m, m.t, Vb(m, k + 1), prec);
   if (o.fast && (n % 2) == 0) {
-    mgs_coop(m, k);
+    gram_schmidt(m, k);
     return;
   }
   for (int v = 0; v <= k; v++) {
@@ -793,7 +705,6 @@ void arnoldi_step_graph(DevMesh &m, const Ops &o, int k, int prec)
   }
   cudaGraphExec_t &ge = m.arnoldi[prec][fo][k];
   if (!ge) {
-    mgs_coop_prepare(m);
     const unsigned long long before = kfun3d_launch_count();
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(m.stream, cudaStreamCaptureModeThreadLocal);
@@ -1634,7 +1545,7 @@ extern "C" double kfun3d_time_kernel(GEOMETRY *g, int which, int reps)
       case 5: arnoldi_step(*m, o, 15, prec); break;
       case 6:
         if (o.fast) {
-          mgs_coop(*m, 15);
+          gram_schmidt(*m, 15);
           break;
         }
         for (int vv = 0; vv <= 15; vv++) {
