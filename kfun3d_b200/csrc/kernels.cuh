@@ -122,19 +122,41 @@ __device__ __forceinline__ double4 recon(double4 q, double4 gx, double4 gy, doub
 __device__ __forceinline__ double4 edge_flux(double4 geo, double4 sL, double4 sR)
 {
   const double xn = geo.x, yn = geo.y, zn = geo.z, ln = geo.w;
-  const Frame f = tangents(xn, yn, zn);
   double ubarL = xn * sL.y; ubarL += yn * sL.z; ubarL += zn * sL.w;
   double ubarR = xn * sR.y; ubarR += yn * sR.z; ubarR += zn * sR.w;
   const double u = 0.5 * (sL.y + sR.y);
   const double v = 0.5 * (sL.z + sR.z);
   const double w = 0.5 * (sL.w + sR.w);
   double ubar = xn * u; ubar += yn * v; ubar += zn * w;
-  const Phi ph = phis(xn, yn, zn, u, v, w, ubar, f);
   const double c2 = ubar * ubar + KB;
   const double c = sqrt(c2);
   const double e12 = fabs(ubar), e3 = fabs(ubar + c), e4 = fabs(ubar - c);
   const double dp = sR.x - sL.x, du = sR.y - sL.y, dv = sR.z - sL.z, dw = sR.w - sL.w;
 
+#if KF_FAST
+  // |A| = |ubar| I + (|ubar + c| - |ubar|) r3 l3^T + (|ubar - c| - |ubar|) r4 l4^T:
+  // the two tangential waves share the eigenvalue ubar, so their part is what
+  // the acoustic ones leave of the identity and no tangent frame is formed
+  // (about 165 instead of 260 FP64 operations an edge: the edge pass is bound
+  // by its gathers on large meshes, edges + nodes at 120^3 540 -> 522 us)
+  const double nd = xn * du + yn * dv + zn * dw, hc2 = 0.5 / c2;
+  const double a3 = (e3 - e12) * (hc2 * ((c - ubar) * INV_B * dp + nd));
+  const double a4 = (e4 - e12) * (hc2 * (nd - (c + ubar) * INV_B * dp));
+  const double su = a3 * (ubar + c) + a4 * (ubar - c), sb = KB * (a3 + a4);
+  const double t1 = e12 * dp + c * KB * (a3 - a4);
+  const double t2 = e12 * du + u * su + xn * sb;
+  const double t3 = e12 * dv + v * su + yn * sb;
+  const double t4 = e12 * dw + w * su + zn * sb;
+  const double hl = 0.5 * ln, ps = sL.x + sR.x;
+  double4 res;
+  res.x = hl * (KB * (ubarL + ubarR) - t1);
+  res.y = hl * (sL.y * ubarL + sR.y * ubarR + xn * ps - t2);
+  res.z = hl * (sL.z * ubarL + sR.z * ubarR + yn * ps - t3);
+  res.w = hl * (sL.w * ubarL + sR.w * ubarR + zn * ps - t4);
+  return res;
+#else
+  const Frame f = tangents(xn, yn, zn);
+  const Phi ph = phis(xn, yn, zn, u, v, w, ubar, f);
   double ti11 = u * ph.p4; ti11 += v * ph.p5; ti11 += w * ph.p6; ti11 = div_b(-ti11);
   double ti21 = u * ph.p7; ti21 += v * ph.p8; ti21 += w * ph.p9; ti21 = div_b(-ti21);
   double ti31 = 0.5 * (c - ubar); ti31 = div_b(ti31);
@@ -144,19 +166,11 @@ __device__ __forceinline__ double4 edge_flux(double4 geo, double4 sL, double4 sR
   double dv2 = ti21 * dp; dv2 += ph.p7 * du; dv2 += ph.p8 * dv; dv2 += ph.p9 * dw;
   double dv3 = 2.0 * ti31 * dp; dv3 += xn * du; dv3 += yn * dv; dv3 += zn * dw;
   double dv4 = 2.0 * ti41 * dp; dv4 += xn * du; dv4 += yn * dv; dv4 += zn * dw;
-#if KF_FAST
-  const double ic2 = 1.0 / c2;
-  dv1 *= ic2;
-  dv2 *= ic2;
-  dv3 *= 0.5 * ic2;
-  dv4 *= 0.5 * ic2;
-#else
   dv1 /= c2;
   dv2 /= c2;
   const double hc2 = 0.5 / c2;
   dv3 *= hc2;
   dv4 *= hc2;
-#endif
   const double r13 = c * KB;
   double r23 = u * (ubar + c); r23 += xn * KB;
   double r33 = v * (ubar + c); r33 += yn * KB;
@@ -188,6 +202,7 @@ __device__ __forceinline__ double4 edge_flux(double4 geo, double4 sL, double4 sR
   res.z = 0.5 * (fp3 + fm3 - ln * t3);
   res.w = 0.5 * (fp4 + fm4 - ln * t4);
   return res;
+#endif
 }
 
 // Characteristic far-field flux at one node, src/flux.c:552-778.
@@ -797,7 +812,6 @@ __global__ void k_timestep_boundary(uint32_t nb, const uint32_t *__restrict__ bn
 __device__ __forceinline__ void edge_jacobians(double4 geo, double4 qa, double4 qb, double *v0, double *v1)
 {
   const double xn = geo.x, yn = geo.y, zn = geo.z, ln = geo.w;
-  const Frame f = tangents(xn, yn, zn);
   const double uL = qa.y, vL = qa.z, wL = qa.w;
   double ubarL = xn * uL; ubarL += yn * vL; ubarL += zn * wL;
   const double uR = qb.y, vR = qb.z, wR = qb.w;
@@ -807,17 +821,7 @@ __device__ __forceinline__ void edge_jacobians(double4 geo, double4 qa, double4 
   const double c2 = ubar * ubar + KB;
   const double c = sqrt(c2);
   const double e12 = ln * fabs(ubar), e3 = ln * fabs(ubar + c), e4 = ln * fabs(ubar - c);
-  const Phi ph = phis(xn, yn, zn, u, v, w, ubar, f);
   const double c2inv = 1.0 / c2;
-  double y1[4], y2[4], y3[4], y4[4];   // rows of T^-1, columns p,u,v,w
-  double t;
-  t = u * ph.p4; t += v * ph.p5; t += w * ph.p6; y1[0] = div_b(-c2inv * t);
-  t = u * ph.p7; t += v * ph.p8; t += w * ph.p9; y2[0] = div_b(-c2inv * t);
-  t = c2inv * (c - ubar); y3[0] = div_b(0.5 * t);
-  t = c2inv * (c + ubar); y4[0] = div_b(-0.5 * t);
-  y1[1] = c2inv * ph.p4; y2[1] = c2inv * ph.p7; y3[1] = c2inv * 0.5 * xn; y4[1] = c2inv * 0.5 * xn;
-  y1[2] = c2inv * ph.p5; y2[2] = c2inv * ph.p8; y3[2] = c2inv * 0.5 * yn; y4[2] = c2inv * 0.5 * yn;
-  y1[3] = c2inv * ph.p6; y2[3] = c2inv * ph.p9; y3[3] = c2inv * 0.5 * zn; y4[3] = c2inv * 0.5 * zn;
   const double t13 = c * KB;
   double t23 = u * (ubar + c); t23 += xn * KB;
   double t33 = v * (ubar + c); t33 += yn * KB;
@@ -827,6 +831,38 @@ __device__ __forceinline__ void edge_jacobians(double4 geo, double4 qa, double4 
   double t34 = v * (ubar - c); t34 += yn * KB;
   double t44 = w * (ubar - c); t44 += zn * KB;
   double a[4][4];   // |A| = T |Lambda| T^-1, src/fill.c:367-439
+#if KF_FAST
+  // as in edge_flux: |ubar| I plus the two acoustic waves' rank-one terms,
+  // whose left vectors differ in their pressure entry only (the fill's row
+  // kernel: 152 -> 128 registers; 40^3 FP32 86 -> 66 us, 70^3 FP64 385 -> 363,
+  // 120^3 FP64 2061 -> 1980)
+  {
+    const double h3 = e3 - e12, h4 = e4 - e12, hc = 0.5 * c2inv;
+    const double l3 = hc * INV_B * (c - ubar), l4 = -hc * INV_B * (c + ubar);
+    const double nx = hc * xn, ny = hc * yn, nz = hc * zn;
+    const double r3[4] = {h3 * t13, h3 * t23, h3 * t33, h3 * t43}, r4[4] = {h4 * t14, h4 * t24, h4 * t34, h4 * t44};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const double s = r3[i] + r4[i];
+      a[i][0] = r3[i] * l3 + r4[i] * l4;
+      a[i][1] = s * nx;
+      a[i][2] = s * ny;
+      a[i][3] = s * nz;
+      a[i][i] += e12;
+    }
+  }
+#else
+  const Frame f = tangents(xn, yn, zn);
+  const Phi ph = phis(xn, yn, zn, u, v, w, ubar, f);
+  double y1[4], y2[4], y3[4], y4[4];   // rows of T^-1, columns p,u,v,w
+  double t;
+  t = u * ph.p4; t += v * ph.p5; t += w * ph.p6; y1[0] = div_b(-c2inv * t);
+  t = u * ph.p7; t += v * ph.p8; t += w * ph.p9; y2[0] = div_b(-c2inv * t);
+  t = c2inv * (c - ubar); y3[0] = div_b(0.5 * t);
+  t = c2inv * (c + ubar); y4[0] = div_b(-0.5 * t);
+  y1[1] = c2inv * ph.p4; y2[1] = c2inv * ph.p7; y3[1] = c2inv * 0.5 * xn; y4[1] = c2inv * 0.5 * xn;
+  y1[2] = c2inv * ph.p5; y2[2] = c2inv * ph.p8; y3[2] = c2inv * 0.5 * yn; y4[2] = c2inv * 0.5 * yn;
+  y1[3] = c2inv * ph.p6; y2[3] = c2inv * ph.p9; y3[3] = c2inv * 0.5 * zn; y4[3] = c2inv * 0.5 * zn;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     double s = e3 * t13 * y3[j];
@@ -839,6 +875,7 @@ __device__ __forceinline__ void edge_jacobians(double4 geo, double4 qa, double4 
     s = e12 * f.z1 * y1[j]; s += e12 * f.z2 * y2[j]; s += e3 * t43 * y3[j]; s += e4 * t44 * y4[j];
     a[3][j] = s;
   }
+#endif
   const double lb = ln * KB, lx = ln * xn, ly = ln * yn, lz = ln * zn;
   v0[0] = 0.5 * a[0][0];
   v0[4] = 0.5 * (lx + a[1][0]);
