@@ -437,7 +437,7 @@ static void release_device(MatrixHandle *h)
   for (void *p : {m->pk_buf, (void *)m->flow_buf, (void *)m->flow_ctl})
     if (p) cudaFree(p);
   void *ptrs[] = {m->col, m->egeo, m->xyz, m->inc_ptr, m->inc_oth, m->inc_edge, m->inc_blk, m->inc_w, m->wf_nodes,
-                  m->wf_n, m->s_n, m->f_n, m->bnd_of, m->bnd_node, m->bnd_ptr, m->bnd_ent, m->ia, m->ja,
+                  m->wf_n, m->s_n, m->f_n, m->bnd_of, m->bndp, m->f_node, m->fres, m->bnd_node, m->bnd_ptr, m->bnd_ent, m->ia, m->ja,
                   m->diag, m->tblk, m->lpos, m->last_lower, m->lev_l, m->lev_u, m->A, m->lslot, m->dinv,
                   m->Af, m->dinvf, m->q, m->r, m->gx, m->gy, m->gz, m->cdt, m->w, m->t, m->x, m->rhs, m->V,
                   m->red, m->scal, m->forces, m->dscr, m->status, m->flags, m->ticket, m->gs_part, m->lsq_coef,
@@ -827,6 +827,11 @@ DevMesh *kf_device(const GEOMETRY *g)
     }
     m->nb = (uint32_t)nodes.size();
     KF_CUDA(upload(&m->bnd_of, of.data(), N));
+    std::vector<uint32_t> ofp(N);
+    for (uint32_t i = 0; i < N; i++) ofp[i] = of[ord[i]];
+    KF_CUDA(upload(&m->bndp, ofp.data(), N));
+    KF_CUDA(upload(&m->f_node, g->b->f->nptr, m->Nf));
+    KF_CUDA(cudaMalloc(&m->fres, std::max<size_t>(m->Nf, 1) * sizeof(double4)));
     KF_CUDA(upload(&m->bnd_node, nodes.data(), nodes.size()));
     KF_CUDA(upload(&m->bnd_ptr, bptr.data(), bptr.size()));
     KF_CUDA(upload(&m->bnd_ent, bent.data(), bent.size()));

@@ -313,6 +313,9 @@ struct DevMesh {
   uint32_t *col = nullptr;        // [ncol+1] wall-face colour offsets
   double *s_n = nullptr;          // [3 Ns] wall-node normals
   double *f_n = nullptr;          // [3 Nf] far-field node normals
+  uint32_t *f_node = nullptr;     // [Nf] far-field nodes
+  double4 *fres = nullptr;        // [Nf] their fluxes (two-pass residual)
+  uint32_t *bndp = nullptr;       // [N] bnd_of of the node visited at each position
   uint32_t nb = 0;                // boundary nodes
   uint32_t *bnd_of = nullptr;     // [N] position in bnd_node, or ~0
   uint32_t *bnd_node = nullptr;   // [nb]
@@ -423,6 +426,12 @@ void kfun3d_reset_launch_count_by(unsigned long long n);   // undo counts taken 
 // a wait that gave up).
 cudaError_t kf_flow_reset(DevMesh &m);
 
+// Jacobian-vector product: the residual and the state it is taken at, and the
+// device scalars (|x|, h).
+struct JvArgs {
+  const double *r, *q, *scal;
+};
+
 // Kernel families, one set per arithmetic mode (kernels_exact.cu, kernels_fast.cu).
 #define KF_DECLARE_KERNELS(NS)                                                          \
   namespace NS {                                                                        \
@@ -437,8 +446,7 @@ cudaError_t kf_flow_reset(DevMesh &m);
   void sptrsv_flags(DevMesh &m, const double *b, double *x, int precision, uint32_t *flags); \
   int lsq_setup(DevMesh &m);                                                            \
   void gradient_to_mesh_order(DevMesh &m);                                              \
-  void jv_combine(DevMesh &m, double *y, const double *r, const double *w,              \
-                  const double *q, const double *scal, int ia);                          \
+  void residual_jv(DevMesh &m, const double *w, double *y, int first_order, double u, double v, const JvArgs &jv); \
   }
 KF_DECLARE_KERNELS(kf_exact)
 KF_DECLARE_KERNELS(kf_fast)

@@ -252,6 +252,15 @@ __device__ __forceinline__ double4 farfield_flux(double U, double V, double fx, 
   return o;
 }
 
+// One 32-byte record in a single 256-bit read-only load (records are 32-byte
+// aligned: elements of cudaMalloc'd arrays).
+__device__ __forceinline__ double4 ldg4(const double4 *p)
+{
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+
 // ------------------------------------------------------------------ TMA bulk staging
 
 // 1-D bulk copies (cp.async.bulk, the TMA engine's untiled path) into shared
@@ -540,11 +549,29 @@ __global__ void __launch_bounds__(256, 4) k_gradient4(uint32_t N, const uint32_t
   const double qn = q[4 * (size_t)n + r];
   double ax = 0.0, ay = 0.0, az = 0.0;
   const uint32_t k1 = inc_ptr[p + 1];
-  for (uint32_t k = inc_ptr[p]; k < k1; k++) {
-    const double dq = q[4 * (size_t)inc_oth[k] + r] - qn;
-    ax += inc_w[k] * dq;
-    ay += inc_w[ninc + k] * dq;
-    az += inc_w[2 * (size_t)ninc + k] * dq;
+  uint32_t k = inc_ptr[p];
+  // four incidences' loads in flight, added in edge order
+  for (; k + 4 <= k1; k += 4) {
+    double dq[4], w[3][4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      dq[u] = q[4 * (size_t)inc_oth[k + u] + r];
+#pragma unroll
+      for (int d = 0; d < 3; d++) w[d][u] = inc_w[d * (size_t)ninc + k + u];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const double d = dq[u] - qn;
+      ax += w[0][u] * d;
+      ay += w[1][u] * d;
+      az += w[2][u] * d;
+    }
+  }
+  for (; k < k1; k++) {
+    const double d = q[4 * (size_t)inc_oth[k] + r] - qn;
+    ax += inc_w[k] * d;
+    ay += inc_w[ninc + k] * d;
+    az += inc_w[2 * (size_t)ninc + k] * d;
   }
   gx[4 * (size_t)n + r] = ax;
   gy[4 * (size_t)n + r] = ay;
@@ -631,21 +658,35 @@ __global__ void __launch_bounds__(128) k_residual(uint32_t N, const uint32_t *__
 // edges are then close in space (their end points' data is shared in L2 and
 // L1), and eoff / in1_ptr are indexed by visit position, in1_edge holds
 // storage positions.
+// The first nfb blocks evaluate the characteristic flux of the far-field nodes
+// (fq: the state in the mesh's numbering), which the node pass adds: its long
+// chain of square roots and divisions then runs beside the edges instead of
+// in a launch of its own after them (edges, nodes and boundary at 25^3: 28.5 ->
+// 18.5 us).  End points are read as 256-bit records.  Seven CTAs an SM (72
+// registers): 522 us with the node pass at 120^3, 532 with five, 582 with six.
 template <bool FIRST_ORDER>
-__global__ void __launch_bounds__(128) k_flux_edges(uint32_t E, const uint32_t *__restrict__ n0,
+__global__ void __launch_bounds__(128, 7) k_flux_edges(uint32_t E, const uint32_t *__restrict__ n0,
                                                     const uint32_t *__restrict__ n1,
                                                     const double4 *__restrict__ egeo,
                                                     const double4 *__restrict__ xyz,
                                                     const double4 *__restrict__ q,
                                                     const double4 *__restrict__ gx,
                                                     const double4 *__restrict__ gy,
-                                                    const double4 *__restrict__ gz, double4 *__restrict__ res)
+                                                    const double4 *__restrict__ gz, double4 *__restrict__ res,
+                                                    uint32_t nfb, uint32_t Nf, const uint32_t *__restrict__ f_node,
+                                                    const double *__restrict__ f_n, const double4 *__restrict__ fq,
+                                                    double U, double V, double4 *__restrict__ fres)
 {
-  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x < nfb) {
+    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f < Nf) fres[f] = farfield_flux(U, V, f_n[3 * f], f_n[3 * f + 1], f_n[3 * f + 2], fq[f_node[f]]);
+    return;
+  }
+  const uint32_t e = (blockIdx.x - nfb) * blockDim.x + threadIdx.x;
   if (e >= E) return;
   const uint32_t a = n0[e], o = n1[e];
-  const double4 geo = egeo[e];
-  const double4 qa = q[a], xa = xyz[a], qb = q[o], xb = xyz[o];
+  const double4 geo = ldg4(egeo + e);
+  const double4 qa = ldg4(q + a), xa = ldg4(xyz + a), qb = ldg4(q + o), xb = ldg4(xyz + o);
   const double xm = 0.5 * (xa.x + xb.x), ym = 0.5 * (xa.y + xb.y), zm = 0.5 * (xa.z + xb.z);
   double4 sL, sR;
   if (FIRST_ORDER) {
@@ -653,48 +694,85 @@ __global__ void __launch_bounds__(128) k_flux_edges(uint32_t E, const uint32_t *
     sL = recon(qa, z, z, z, xm - xa.x, ym - xa.y, zm - xa.z);
     sR = recon(qb, z, z, z, xm - xb.x, ym - xb.y, zm - xb.z);
   } else {
-    sL = recon(qa, gx[a], gy[a], gz[a], xm - xa.x, ym - xa.y, zm - xa.z);
-    sR = recon(qb, gx[o], gy[o], gz[o], xm - xb.x, ym - xb.y, zm - xb.z);
+    const double4 gxa = ldg4(gx + a), gya = ldg4(gy + a), gza = ldg4(gz + a);
+    const double4 gxb = ldg4(gx + o), gyb = ldg4(gy + o), gzb = ldg4(gz + o);
+    sL = recon(qa, gxa, gya, gza, xm - xa.x, ym - xa.y, zm - xa.z);
+    sR = recon(qb, gxb, gyb, gzb, xm - xb.x, ym - xb.y, zm - xb.z);
   }
   res[e] = edge_flux(geo, sL, sR);
 }
 
-__global__ void __launch_bounds__(256) k_flux_nodes(uint32_t N, const uint32_t *__restrict__ ord,
-                                                    const uint32_t *__restrict__ in1_ptr,
-                                                    const uint32_t *__restrict__ in1_edge,
-                                                    const uint32_t *__restrict__ eoff,
-                                                    const double4 *__restrict__ res, double4 *__restrict__ r)
-{
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N) return;
-  const uint32_t n = ord[p];
-  double4 acc = make_double4(0, 0, 0, 0);
-  const uint32_t k1 = in1_ptr[p + 1];
-  for (uint32_t k = in1_ptr[p]; k < k1; k++) acc = sub4(acc, res[in1_edge[k]]);
-  const uint32_t e1 = eoff[p + 1];
-  for (uint32_t e = eoff[p]; e < e1; e++) acc = add4(acc, res[e]);
-  r[n] = acc;
-}
-
-// k_flux_nodes with four lanes per node, lane r summing flux component r in
-// the same order (so the same result): a quad reads each edge flux as one
-// 32-byte sector, and four times as many nodes' gathers are in flight.
-__global__ void __launch_bounds__(256) k_flux_nodes4(uint32_t N, const uint32_t *__restrict__ ord,
-                                                     const uint32_t *__restrict__ in1_ptr,
-                                                     const uint32_t *__restrict__ in1_edge,
-                                                     const uint32_t *__restrict__ eoff,
-                                                     const double *__restrict__ res, double *__restrict__ r)
+// The node pass, four lanes per node, lane c summing flux component c in the
+// reference's order: a quad reads each edge flux as one 32-byte sector.  Then,
+// for boundary nodes (bndp[p] their position in the boundary lists, ~0
+// elsewhere), the wall faces by colour (src/flux.c:467-539) and the far-field
+// fluxes (src/flux.c:541-779) in list order.  JV: the sum y is not stored but
+// (y - r + cdt (w - q)) |x| / h, the Jacobian-vector product of
+// src/kernel.c:35-44 (w in visit order when wv is given).
+struct NodePass {
+  const uint32_t *ord, *in1_ptr, *in1_edge, *eoff;
+  const uint32_t *bndp, *bnd_ptr, *bnd_ent, *wf_nodes;
+  const double *wf_n, *fres;
+  const double4 *q;                        // the state, mesh numbering
+  const double *jr, *jw, *jwv, *jq, *jcdt, *jscal;   // JV: r, w, w in visit order or null, q, cdt, (|x|, h)
+};
+template <bool JV>
+__global__ void __launch_bounds__(256, 6) k_flux_nodes4(uint32_t N, NodePass a, const double *__restrict__ res,
+                                                     double *__restrict__ r)
 {
   const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t p = gid >> 2, c = gid & 3;
   if (p >= N) return;
-  const uint32_t n = ord[p];
-  double acc = 0.0;
-  const uint32_t k1 = in1_ptr[p + 1];
-  for (uint32_t k = in1_ptr[p]; k < k1; k++) acc = acc - res[4 * (size_t)in1_edge[k] + c];
-  const uint32_t e1 = eoff[p + 1];
-  for (uint32_t e = eoff[p]; e < e1; e++) acc = acc + res[4 * (size_t)e + c];
-  r[4 * (size_t)n + c] = acc;
+  const uint32_t n = a.ord[p];
+  const size_t own = 4 * (size_t)n + c;
+  double acc = 0.0, jr = 0.0, jw = 0.0, jq = 0.0, jc = 0.0;
+  if (JV) {
+    jr = a.jr[own];
+    jq = a.jq[own];
+    jw = a.jwv ? a.jwv[4 * (size_t)p + c] : a.jw[own];
+    jc = a.jcdt[n];
+  }
+  const uint32_t bo = a.bndp[p];
+  uint32_t k = a.in1_ptr[p];
+  const uint32_t k1 = a.in1_ptr[p + 1], e1 = a.eoff[p + 1];
+  for (; k + 4 <= k1; k += 4) {
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = res[4 * (size_t)a.in1_edge[k + u] + c];
+#pragma unroll
+    for (int u = 0; u < 4; u++) acc = acc - v[u];
+  }
+  for (; k < k1; k++) acc = acc - res[4 * (size_t)a.in1_edge[k] + c];
+  uint32_t e = a.eoff[p];
+  for (; e + 4 <= e1; e += 4) {
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = res[4 * (size_t)(e + u) + c];
+#pragma unroll
+    for (int u = 0; u < 4; u++) acc = acc + v[u];
+  }
+  for (; e < e1; e++) acc = acc + res[4 * (size_t)e + c];
+  if (bo != 0xffffffffu)
+    for (uint32_t b = a.bnd_ptr[bo]; b < a.bnd_ptr[bo + 1]; b++) {
+      const uint32_t ent = a.bnd_ent[b], kind = ent >> 29, idx = ent & 0x1fffffffu;
+      if (kind == 0 && c > 0) {
+        const uint32_t f = idx / 3, corner = idx % 3;
+        const double p1 = a.q[a.wf_nodes[3 * f]].x, p2 = a.q[a.wf_nodes[3 * f + 1]].x,
+                     p3 = a.q[a.wf_nodes[3 * f + 2]].x;
+        double pr;
+        if (corner == 0) { pr = 0.125 * (p2 + p3); pr += 0.75 * p1; }
+        else if (corner == 1) { pr = 0.125 * (p3 + p1); pr += 0.75 * p2; }
+        else { pr = 0.125 * (p1 + p2); pr += 0.75 * p3; }
+        acc += a.wf_n[3 * f + c - 1] * pr;
+      } else if (kind == 2) {
+        acc += a.fres[4 * (size_t)idx + c];
+      }
+    }
+  if (JV) {
+    const double s = a.jscal[0] / a.jscal[1];
+    acc = (acc - jr + jc * (jw - jq)) * s;
+  }
+  r[own] = acc;
 }
 
 // Boundary terms, after all edges: wall faces by colour (src/flux.c:467-539),
@@ -2459,7 +2537,8 @@ void gradient_to_mesh_order(DevMesh &m)
 // Residual of q into r.  With visit-order copies (m.visit) the edge pass
 // reads the state, coordinates and gradients from them: the copy of q made
 // by gradient() for the second-order flux, made here for the first order.
-void residual(DevMesh &m, const double *q, double *r, int first_order, double u, double v)
+// With jv (the two-pass form only) r receives the Jacobian-vector product.
+static void residual_or_jv(DevMesh &m, const double *q, double *r, int first_order, double u, double v, const JvArgs *jv)
 {
   if (m.two_pass) {
     if (first_order) visit_state(m, q);
@@ -2468,18 +2547,35 @@ void residual(DevMesh &m, const double *q, double *r, int first_order, double u,
     const double4 *Q = m.visit ? m.qv : (const double4 *)q;
     const double4 *X = m.visit ? m.xyzv : m.xyz;
     const uint32_t *E0 = m.visit ? m.n0v : m.n0s, *E1 = m.visit ? m.n1v : m.n1;
-    {
+    const uint32_t nfb = blocks(m.Nf, 128);
+    if (nfb + blocks(m.E, 128)) {
       if (first_order)
-        k_flux_edges<true><<<blocks(m.E, 128), 128, 0, m.stream>>>(m.E, E0, E1, m.egeo_s, X, Q, nullptr, nullptr,
-                                                                    nullptr, m.eres);
+        k_flux_edges<true><<<nfb + blocks(m.E, 128), 128, 0, m.stream>>>(
+            m.E, E0, E1, m.egeo_s, X, Q, nullptr, nullptr, nullptr, m.eres, nfb, m.Nf, m.f_node, m.f_n,
+            (const double4 *)q, u, v, m.fres);
       else
-        k_flux_edges<false><<<blocks(m.E, 128), 128, 0, m.stream>>>(m.E, E0, E1, m.egeo_s, X, Q, G[0], G[1], G[2],
-                                                                     m.eres);
-      k_flux_nodes4<<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, m.ord, m.in1_ptr, m.in1_edge, m.eoff,
-                                                                         (const double *)m.eres, r);
-      kf_count_launch(2);
+        k_flux_edges<false><<<nfb + blocks(m.E, 128), 128, 0, m.stream>>>(
+            m.E, E0, E1, m.egeo_s, X, Q, G[0], G[1], G[2], m.eres, nfb, m.Nf, m.f_node, m.f_n, (const double4 *)q, u, v,
+            m.fres);
+      kf_count_launch();
     }
-  } else if (first_order)
+    NodePass a{m.ord, m.in1_ptr, m.in1_edge, m.eoff, m.bndp, m.bnd_ptr, m.bnd_ent, m.wf_nodes, m.wf_n,
+               (const double *)m.fres, (const double4 *)q, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    if (jv) {
+      a.jr = jv->r;
+      a.jw = q;
+      a.jwv = m.visit ? (const double *)m.qv : nullptr;
+      a.jq = jv->q;
+      a.jcdt = m.cdt;
+      a.jscal = jv->scal;
+      k_flux_nodes4<true><<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, a, (const double *)m.eres, r);
+    } else {
+      k_flux_nodes4<false><<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, a, (const double *)m.eres, r);
+    }
+    kf_count_launch();
+    return;
+  }
+  if (first_order)
     k_residual<true><<<blocks(m.N, 128), 128, 0, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_edge, m.egeo, m.xyz,
                                                             (const double4 *)q, nullptr, nullptr, nullptr,
                                                             (double4 *)r);
@@ -2488,10 +2584,26 @@ void residual(DevMesh &m, const double *q, double *r, int first_order, double u,
                                                              (const double4 *)q, (const double4 *)m.gx,
                                                              (const double4 *)m.gy, (const double4 *)m.gz,
                                                              (double4 *)r);
-  if (!m.two_pass) kf_count_launch();
+  kf_count_launch();
   if (m.nb) {
     k_residual_boundary<<<blocks(m.nb, 64), 64, 0, m.stream>>>(m.nb, m.bnd_node, m.bnd_ptr, m.bnd_ent, m.wf_nodes,
                                                                m.wf_n, m.f_n, (const double4 *)q, (double4 *)r, u, v);
+    kf_count_launch();
+  }
+}
+
+void residual(DevMesh &m, const double *q, double *r, int first_order, double u, double v)
+{
+  residual_or_jv(m, q, r, first_order, u, v, nullptr);
+}
+
+// y = (F(w) - r + cdt (w - q)) scal[0] / scal[1] (src/kernel.c:33-44), the
+// gradient of w formed before
+void residual_jv(DevMesh &m, const double *w, double *y, int first_order, double u, double v, const JvArgs &jv)
+{
+  residual_or_jv(m, w, y, first_order, u, v, m.two_pass ? &jv : nullptr);
+  if (!m.two_pass) {
+    k_jv_combine<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, y, jv.r, w, jv.q, m.cdt, jv.scal, 0);
     kf_count_launch();
   }
 }
@@ -2991,12 +3103,6 @@ void sptrsv_flags(DevMesh &m, const double *b, double *x, int precision, uint32_
     launch((const void *)k_trsv_syncfree<float, true>, m.desc_u, &eU);
   }
   kf_count_launch(2);
-}
-
-void jv_combine(DevMesh &m, double *y, const double *r, const double *w, const double *q, const double *scal, int ia)
-{
-  k_jv_combine<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, y, r, w, q, m.cdt, scal, ia);
-  kf_count_launch();
 }
 
 }  // namespace KF_NS

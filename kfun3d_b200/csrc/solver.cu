@@ -542,9 +542,9 @@ struct Ops {
     }
     fast ? kf_fast::sptrsv(m, b, x, p) : kf_exact::sptrsv(m, b, x, p);
   }
-  void jv_combine(DevMesh &m, double *y, const double *r, const double *w, const double *q) const
+  void residual_jv(DevMesh &m, const double *w, double *y, int fo, double u, double v, const JvArgs &jv) const
   {
-    fast ? kf_fast::jv_combine(m, y, r, w, q, m.scal, S_XN) : kf_exact::jv_combine(m, y, r, w, q, m.scal, S_XN);
+    fast ? kf_fast::residual_jv(m, w, y, fo, u, v, jv) : kf_exact::residual_jv(m, w, y, fo, u, v, jv);
   }
 };
 
@@ -594,8 +594,11 @@ void dev_jacvec(DevMesh &m, const Ops &o, const double *x, double *y)
     k_jv_shift<<<nblk(n, 256), 256, 0, m.stream>>>(n, m.scal, x, m.q, m.w, o.fast);
   }
   kf_count_launch(2);
-  dev_residual(m, o, m.w, y);
-  o.jv_combine(m, y, m.r, m.w, m.q);
+  double u, v;
+  kfun3d_get_freestream(&u, &v);
+  const int fo = kf_first_order();
+  if (!fo) o.gradient(m, m.w);
+  o.residual_jv(m, m.w, y, fo, u, v, JvArgs{m.r, m.q, m.scal + S_XN});
 }
 
 void dev_axpy(DevMesh &m, double a, const double *x, double *y, bool fast)
