@@ -846,6 +846,13 @@ DevMesh *kf_device(const GEOMETRY *g)
   m->lev_u_ptr = p.lev_u_ptr;
   m->nlev_l = (uint32_t)p.lev_l_ptr.size() - 1;
   m->nlev_u = (uint32_t)p.lev_u_ptr.size() - 1;
+  m->max_lower = kf_max_lower(p);
+  {
+    // ILU(0) levels: rows staged through shared memory (default), or "pairs",
+    // the kernels for rows longer than that holds
+    const char *env = getenv("KFUN3D_ILU");
+    m->ilu_rows = !(env && strcmp(env, "pairs") == 0);
+  }
   const size_t nb16 = 16 * (size_t)m->nnz;
   KF_CUDA(cudaMalloc(&m->A, nb16 * sizeof(double)));
   KF_CUDA(cudaMalloc(&m->Af, nb16 * sizeof(float)));
@@ -962,6 +969,7 @@ DevMesh *kf_device(const GEOMETRY *g)
     s0.lev_l = m->lev_l; s0.lev_u = m->lev_u; s0.lev_ptr_d = m->lev_ptr_d;
     s0.lev_l_ptr = m->lev_l_ptr; s0.lev_u_ptr = m->lev_u_ptr;
     s0.nlev_l = m->nlev_l; s0.nlev_u = m->nlev_u;
+    s0.max_lower = m->max_lower;
     s0.desc_l = m->desc_l; s0.desc_u = m->desc_u;
     s0.trsv_mode = m->trsv_mode;
     m->pk[0] = s0.pk[0];

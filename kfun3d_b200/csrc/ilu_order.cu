@@ -62,6 +62,7 @@ void activate(DevMesh &m, const IluSet &s)
   m.pk[0] = s.pk[0];
   m.pk[1] = s.pk[1];
   m.row_node = s.row_node;
+  m.max_lower = s.max_lower;
 }
 
 // Tiles of the tile-major order (KFUN3D_ILU_PERM=tiles): columns along the
@@ -279,6 +280,7 @@ int build_spatial(DevMesh &m, const GEOMETRY *g)
   s.lev_u_ptr = p.lev_u_ptr;
   s.nlev_l = (uint32_t)p.lev_l_ptr.size() - 1;
   s.nlev_u = (uint32_t)p.lev_u_ptr.size() - 1;
+  s.max_lower = kf_max_lower(p);
   {
     std::vector<uint32_t> lp(p.lev_l_ptr);
     lp.insert(lp.end(), p.lev_u_ptr.begin(), p.lev_u_ptr.end());

@@ -207,6 +207,7 @@ struct IluSet {
   uint32_t nlev_l = 0, nlev_u = 0;
   uint4 *desc_l = nullptr, *desc_u = nullptr;
   int trsv_mode = 4;
+  uint32_t max_lower = 0;          // lower blocks of the row that has most
   uint32_t *fill_blk = nullptr;    // [2E] block of (node, other) per incidence (CSR order)
   uint32_t *fill_diag = nullptr;   // [N] diagonal block of each node
   uint32_t *fill_last = nullptr;   // [N] the node's row's last-touched lower block (or ~0)
@@ -214,6 +215,14 @@ struct IluSet {
   uint32_t *row_node = nullptr;    // [N] node of each matrix row (null: the identity)
   PackedSweep pk[2];               // packed level schedule (trsv_mode 8)
 };
+
+// Lower blocks of the row that has most.
+inline uint32_t kf_max_lower(const HostPattern &p)
+{
+  uint32_t n = 0;
+  for (size_t i = 0; i < p.n; i++) n = std::max(n, p.diag[i] - p.ia[i]);
+  return n;
+}
 
 // Level-slot descriptors of both sweeps, (row, first block, end block, 0):
 // the lower sweep's blocks left of the diagonal, the upper sweep's right of
@@ -325,6 +334,8 @@ struct DevMesh {
   uint32_t *ia = nullptr, *ja = nullptr, *diag = nullptr, *tblk = nullptr;
   uint32_t *lpos = nullptr, *last_lower = nullptr;
   uint32_t nlev_l = 0, nlev_u = 0;
+  uint32_t max_lower = 0;         // lower blocks of the row that has most
+  bool ilu_rows = true;           // ILU(0) levels with staged rows (k_ilu_rows; KFUN3D_ILU=pairs: not)
   std::vector<uint32_t> lev_l_ptr, lev_u_ptr;   // host copies of level offsets
   uint32_t *lev_l = nullptr, *lev_u = nullptr;
   uint32_t *pair_ptr = nullptr;   // [nnz+1]

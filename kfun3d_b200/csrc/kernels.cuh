@@ -1208,6 +1208,24 @@ __device__ __forceinline__ double gemm_lane(double a, double b, int lane16, unsi
   return s;
 }
 
+__device__ __forceinline__ float gemm_lane_f(float a, float b, int lane16, unsigned mask, int base)
+{
+  const int r = lane16 >> 2, c = lane16 & 3;
+  float s = 0.0f;
+#pragma unroll
+  for (int t = 0; t < 4; t++) s += __shfl_sync(mask, a, base + 4 * r + t) * __shfl_sync(mask, b, base + 4 * t + c);
+  return s;
+}
+
+__device__ __forceinline__ double gemm_any(double a, double b, int l16, unsigned mask, int base)
+{
+  return gemm_lane(a, b, l16, mask, base);
+}
+__device__ __forceinline__ float gemm_any(float a, float b, int l16, unsigned mask, int base)
+{
+  return gemm_lane_f(a, b, l16, mask, base);
+}
+
 // One level of the ILU(0) sweep of matrix/ilu.cpp:49-97, 16 lanes per row.
 // For block (i,k) the lanes walk row i's lower columns plus the diagonal
 // against column k of U (row k's lower columns plus k, through tblk),
@@ -1332,6 +1350,163 @@ __global__ void __launch_bounds__(128) k_ilu_level_pairs(uint32_t nrows, const u
   }
 }
 
+// The same level of the sweep with a row's operands on their way before they
+// are used (both precisions; every row's lower blocks fit KF_ILU_LMAX).  The
+// products of a row's blocks are one run of `pairs`: its U blocks come through
+// a ring of two batches of 16 in shared memory (cp.async, one batch ahead of
+// the products), its L blocks stay in shared memory as they are formed, and
+// the next block, its column's inverse and its product count are loaded a
+// block ahead.  What a row then waits for is the arithmetic of its own chain,
+// not four dependent loads per block.  Everything that earlier levels do not
+// write is loaded before the previous level's grid has finished
+// (griddepcontrol.wait).  FP64: arithmetic of k_ilu_level_pairs (the last
+// product subtracted and added back, with the row's persistent L slot as its
+// L factor); FP32: that of k_ilu_level_pairs_f32 (no last product).
+// Bound by the instructions of 16-lane products at 16 to 24 warps an SM (the
+// FP64 ring and L blocks take 6 KB a row).  Whole factorisation with the packed
+// copy, pair kernels / this: 10^3 FP64 650 / 394 us, 25^3 FP64 1105 / 575, 40^3
+// FP32 spatial 890 / 608, 70^3 FP64 3131 / 2730, 120^3 FP32 spatial 6.68 / 5.80
+// ms, 120^3 FP64 11.9 / 11.5 ms.
+constexpr uint32_t KF_ILU_LMAX = 32;   // lower blocks of a row held on chip, at most
+__device__ __forceinline__ void load4(const double *p, double &a, double &b, double &c, double &d)
+{
+  const double2 u = reinterpret_cast<const double2 *>(p)[0], v = reinterpret_cast<const double2 *>(p)[1];
+  a = u.x; b = u.y; c = v.x; d = v.y;
+}
+__device__ __forceinline__ void load4(const float *p, float &a, float &b, float &c, float &d)
+{
+  const float4 v = *reinterpret_cast<const float4 *>(p);
+  a = v.x; b = v.y; c = v.z; d = v.w;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 6) k_ilu_rows(uint32_t nrows, const uint32_t *__restrict__ rows,
+                                                  const uint32_t *__restrict__ ia, const uint32_t *__restrict__ ja,
+                                                  const uint32_t *__restrict__ diag,
+                                                  const uint32_t *__restrict__ pair_ptr,
+                                                  const uint2 *__restrict__ pairs, const uint32_t *__restrict__ lpos,
+                                                  T *A, double *lslot, T *dinv, int *__restrict__ status,
+                                                  uint32_t lmax)
+{
+  constexpr bool D = sizeof(T) == 8;
+  constexpr int W = sizeof(T);        // 16-byte words of a block
+  extern __shared__ __align__(128) unsigned char smem[];   // per row: the ring, lmax L blocks and the identity
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t grp = blockIdx.x * 8 + (threadIdx.x >> 4);
+  const int lane = threadIdx.x & 31, l16 = lane & 15, base = lane & 16, r = l16 >> 2, c = l16 & 3;
+  const unsigned mask = 0xffffu << base;
+  if (grp >= nrows) return;
+  T *ring = reinterpret_cast<T *>(smem) + (threadIdx.x >> 4) * (size_t)(512 + 16 * (lmax + 1));
+  T *lrow = ring + 512;
+  const uint32_t i = rows[grp];
+  const uint32_t j0 = ia[i], j1 = ia[i + 1], nl = diag[i] - j0, lp = lpos[i];
+  const uint32_t p0 = pair_ptr[j0], np = pair_ptr[j1] - p0;
+  auto batch = [&](uint32_t b) -> uint2 {   // the row's products 16 b + l16
+    const uint32_t q = 16 * b + l16;
+    return q < np ? pairs[p0 + q] : make_uint2(0xffffffffu, 0xffffffffu);
+  };
+  auto fetch = [&](const uint2 &pr, int slot) {   // their U blocks
+#pragma unroll
+    for (int q = 0; q < W; q++) {
+      const int w = q * 16 + l16;
+      const uint32_t y = __shfl_sync(mask, pr.y, base + w / W);
+      if (y != 0xffffffffu) {
+        const unsigned dst = smem_addr(ring + 256 * slot) + 16u * (unsigned)w;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                     "l"(reinterpret_cast<const unsigned char *>(A + 16 * (size_t)y) + 16 * (w % W))
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint2 pc = batch(0), pn = batch(1), pnn = batch(2);
+  if (D)
+    for (uint32_t q = 0; q < nl; q++) lrow[16 * q + l16] = (T)lslot[16 * (size_t)(lp + q) + l16];
+  lrow[16 * lmax + l16] = r == c ? T(1) : T(0);
+  uint32_t j = j0, k = ja[j0], kn = j0 + 1 < j1 ? ja[j0 + 1] : i;
+  uint32_t pe = pair_ptr[j0 + 1] - p0, pen = j0 + 1 < j1 ? pair_ptr[j0 + 2] - p0 : 0u;
+  T a = A[16 * (size_t)j0 + l16], an = j0 + 1 < j1 ? A[16 * (size_t)(j0 + 1) + l16] : T(0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  fetch(pc, 0);
+  fetch(pn, 1);
+  T dk = k < i ? __ldcg(dinv + 16 * (size_t)k + l16) : T(0);
+  T dn = kn < i ? __ldcg(dinv + 16 * (size_t)kn + l16) : T(0);
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncwarp(mask);
+  uint32_t cur = 0, bb = 0;   // the block's first product; the batch it is in
+  for (; j < j1; j++) {
+    const uint32_t cnt = D ? pe - cur : pe - cur - 1;
+    T d = T(0);
+    for (uint32_t q = 0; q < cnt; q += 4) {   // four products side by side
+      const uint32_t f = cur + q, n = min(cnt - q, 4u);
+      while ((f >> 4) != bb) {
+        __syncwarp(mask);   // the batch before is used up
+        bb++;
+        pc = pn;
+        pn = pnn;
+        fetch(pn, (bb + 1) & 1);
+        pnn = batch(bb + 2);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp(mask);
+      }
+      if (((f + n - 1) >> 4) != bb) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp(mask);
+      }
+      T e[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const uint32_t g = f + min((uint32_t)u, n - 1);
+        const uint32_t x = __shfl_sync(mask, (g >> 4) == bb ? pc.x : pn.x, base + (int)(g & 15));
+        const T *ub = ring + 16 * (g & 31) + c;
+        T l0, l1, l2, l3;
+        load4(lrow + 16 * (x == 0xffffffffu ? lmax : x - lp) + 4 * r, l0, l1, l2, l3);
+        T s = T(0);
+        s += l0 * ub[0];
+        s += l1 * ub[4];
+        s += l2 * ub[8];
+        s += l3 * ub[12];
+        e[u] = s;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if ((uint32_t)u < n) {
+          d = e[u];
+          if (D) a = T(-1) * d + a;
+          else a -= d;
+        }
+    }
+    if (D) a = T(1) * d + a;
+    if (k < i) {
+      const T lv = gemm_any(a, dk, l16, mask, base);
+      lrow[16 * (j - j0) + l16] = lv;
+      if (D) lslot[16 * (size_t)(lp + (j - j0)) + l16] = (double)lv;
+      else A[16 * (size_t)j + l16] = lv;
+      __syncwarp(mask);
+    } else {
+      A[16 * (size_t)j + l16] = a;
+      if (k == i) {
+        // the inverse of the row's diagonal block, entry l on lane l
+        const double inv = inv4_lane((double)a, l16, mask, base);
+        dinv[16 * (size_t)i + l16] = (T)inv;
+        if (__any_sync(mask, !isfinite(inv)) && l16 == 0) atomicExch(status, KFUN3D_ERR_PIVOT);
+      }
+    }
+    cur = pe;
+    k = kn;
+    pe = pen;
+    a = an;
+    dk = dn;
+    if (j + 2 < j1) {
+      kn = ja[j + 2];
+      pen = pair_ptr[j + 3] - p0;
+      an = A[16 * (size_t)(j + 2) + l16];
+      dn = kn < i ? __ldcg(dinv + 16 * (size_t)kn + l16) : T(0);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 // matrix/ilu.cpp:115-136: the factor over A, lower blocks from the L slots,
 // diagonal blocks inverted.
 __global__ void k_ilu_finish(uint32_t N, const uint32_t *__restrict__ ia, const uint32_t *__restrict__ diag,
@@ -1349,15 +1524,6 @@ __global__ void k_ilu_finish(uint32_t N, const uint32_t *__restrict__ ia, const 
 // FP32 form: plain block ILU(0) in natural order on float blocks (no
 // persistent slots); L(i,k) = (A(i,k) - sum L(i,m) U(m,k)) inv(U(k,k)),
 // U(i,k) = A(i,k) - sum L(i,m) U(m,k), inverses formed in double and rounded.
-__device__ __forceinline__ float gemm_lane_f(float a, float b, int lane16, unsigned mask, int base)
-{
-  const int r = lane16 >> 2, c = lane16 & 3;
-  float s = 0.0f;
-#pragma unroll
-  for (int t = 0; t < 4; t++) s += __shfl_sync(mask, a, base + 4 * r + t) * __shfl_sync(mask, b, base + 4 * t + c);
-  return s;
-}
-
 __global__ void __launch_bounds__(128) k_ilu_level_f32(uint32_t nrows, const uint32_t *__restrict__ rows,
                                                        const uint32_t *__restrict__ ia,
                                                        const uint32_t *__restrict__ ja,
@@ -2684,8 +2850,36 @@ void ilu(DevMesh &m, int precision)
       k_drop_coupling<float><<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, m.ia, m.ja, m.row_node, m.sub_part, m.Af);
     kf_count_launch();
   }
+  // rows staged through shared memory where they fit
+  const bool staged = m.pairs && m.max_lower <= KF_ILU_LMAX && m.ilu_rows;
+  uint32_t lmax = m.max_lower;
+  const size_t smem = 8 * (512 + 16 * (size_t)(lmax + 1)) * (precision == 0 ? sizeof(double) : sizeof(float));
+  if (staged)
+    cudaFuncSetAttribute(precision == 0 ? (const void *)k_ilu_rows<double> : (const void *)k_ilu_rows<float>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   for (uint32_t l = 0; l < m.nlev_l; l++) {
     const uint32_t r0 = m.lev_l_ptr[l], nr = m.lev_l_ptr[l + 1] - r0;
+    if (staged) {
+      const uint32_t *rows = m.lev_l + r0;
+      uint32_t nrows = nr;
+      void *Ap = precision == 0 ? (void *)m.A : (void *)m.Af, *Dp = precision == 0 ? (void *)m.dinv : (void *)m.dinvf;
+      void *args[] = {&nrows,      (void *)&rows,    (void *)&m.ia,   (void *)&m.ja, (void *)&m.diag, (void *)&m.pair_ptr,
+                      (void *)&m.pairs, (void *)&m.lpos, (void *)&Ap, (void *)&m.lslot, (void *)&Dp,  (void *)&status,
+                      &lmax};
+      cudaLaunchConfig_t cfg = {};
+      cfg.dynamicSmemBytes = smem;
+      cfg.gridDim = dim3(blocks(nr, 8));
+      cfg.blockDim = dim3(128);
+      cfg.stream = m.stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = l == 0 ? 0 : 1;   // the first level waits normally for the fill
+      const cudaError_t e = cudaLaunchKernelExC(
+          &cfg, precision == 0 ? (const void *)k_ilu_rows<double> : (const void *)k_ilu_rows<float>, args);
+      if (e != cudaSuccess) kf_set_error(KFUN3D_ERR_CUDA, cudaGetErrorString(e));
+    } else
     if (precision == 0 && m.pairs)
       k_ilu_level_pairs<<<blocks((size_t)nr * 16, 128), 128, 0, m.stream>>>(nr, m.lev_l + r0, m.ia, m.ja, m.diag,
                                                                             m.pair_ptr, m.pairs, m.lpos, m.A,
