@@ -96,26 +96,42 @@ __device__ __forceinline__ void st_chunk(unsigned char *tile, int row, int c, in
 {
   *reinterpret_cast<uint4 *>(tile + kmajor_offset(row, 8 * c, K)) = v;
 }
-// element (f, r) of a transposed 128 x 128 tile (features x rows)
-__device__ __forceinline__ void st_t(unsigned char *tile, int f, int r, uint16_t bits)
-{
-  *reinterpret_cast<uint16_t *>(tile + kmajor_offset(f, r, 128)) = bits;
-}
-__device__ __forceinline__ void st_t_chunk(unsigned char *tile, int f0, int r, uint4 v)
-{
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    st_t(tile, f0 + 2 * i, r, (uint16_t)(w[i] & 0xFFFFu));
-    st_t(tile, f0 + 2 * i + 1, r, (uint16_t)(w[i] >> 16));
-  }
-}
-
 __device__ __forceinline__ void sync_tc()
 {
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
+}
+
+// 32 bytes (32-byte aligned) in one 256-bit read-only load: a gathered row of
+// 64 bytes is two requests instead of four
+__device__ __forceinline__ void ldg32(const uint4 *p, uint4 &a, uint4 &b)
+{
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+      : "l"(p));
+}
+
+// Component c of row r of a tile of 32-float rows in shared memory: a row's
+// 16-byte words are rotated by its index, so that neither threads writing
+// their own rows nor a warp reading one row meet in a bank.
+__device__ __forceinline__ uint32_t row_word(uint32_t r, uint32_t w) { return 32u * r + 4u * ((w + r) & 7u); }
+
+// Sum of component c over rows r0 .. r1 - 1 in row order, from zero; four
+// rows' loads ahead of the additions.
+__device__ __forceinline__ float row_sum(const float *S, uint32_t r0, uint32_t r1, uint32_t c)
+{
+  float sum = 0.f;
+  uint32_t r = r0;
+  for (; r + 4 <= r1; r += 4) {
+    float f[4];
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) f[u] = S[row_word(r + u, c >> 2) + (c & 3u)];
+#pragma unroll
+    for (int u = 0; u < 4; u++) sum += f[u];
+  }
+  for (; r < r1; r++) sum += S[row_word(r, c >> 2) + (c & 3u)];
+  return sum;
 }
 
 // ------------------------------------------------------------ graph
@@ -136,9 +152,17 @@ struct GraphDev {
 
 // ------------------------------------------------------------ gathers (X rows)
 
+// A row's indices and edge features, loaded a tile before the row is gathered
+// through them (edges only).
+struct RowIdx {
+  uint32_t i = 0, j = 0;
+  uint2 e = {0, 0};
+};
+
 struct GatherEnc {   // [x0 (8), 1, 0 x 7]
   const uint4 *x0;
-  __device__ void load(uint32_t i, uint4 *c) const
+  __device__ RowIdx index(uint32_t) const { return RowIdx{}; }
+  __device__ void load(uint32_t i, const RowIdx &, uint4 *c) const
   {
     c[0] = x0[i];
     c[1] = make_uint4(BF16_ONE, 0, 0, 0);
@@ -149,15 +173,21 @@ struct GatherEdge {   // [h_i (32), h_j (32), n (3), a, 1, 0 x 11]
   const uint4 *h;
   const uint32_t *rnode, *oth;
   const uint2 *efeat;
-  __device__ void load(uint32_t r, uint4 *c) const
+  __device__ RowIdx index(uint32_t r) const
   {
-    const uint32_t i = rnode[r], j = oth[r];
-#pragma unroll
-    for (int k = 0; k < 4; k++) c[k] = h[4 * (size_t)i + k];
-#pragma unroll
-    for (int k = 0; k < 4; k++) c[4 + k] = h[4 * (size_t)j + k];
-    const uint2 e = efeat[r];
-    c[8] = make_uint4(e.x, e.y, BF16_ONE, 0);
+    RowIdx x;
+    x.i = rnode[r];
+    x.j = oth[r];
+    x.e = efeat[r];
+    return x;
+  }
+  __device__ void load(uint32_t, const RowIdx &x, uint4 *c) const
+  {
+    ldg32(h + 4 * (size_t)x.i, c[0], c[1]);
+    ldg32(h + 4 * (size_t)x.i + 2, c[2], c[3]);
+    ldg32(h + 4 * (size_t)x.j, c[4], c[5]);
+    ldg32(h + 4 * (size_t)x.j + 2, c[6], c[7]);
+    c[8] = make_uint4(x.e.x, x.e.y, BF16_ONE, 0);
     c[9] = make_uint4(0, 0, 0, 0);
   }
 };
@@ -170,13 +200,14 @@ struct GatherNode {
   const uint4 *msg;
   uint4 *agg_out;
   const uint4 *agg_in;
-  __device__ void load(uint32_t i, uint4 *c) const
+  __device__ RowIdx index(uint32_t) const { return RowIdx{}; }
+  __device__ void load(uint32_t i, const RowIdx &, uint4 *c) const
   {
-#pragma unroll
-    for (int k = 0; k < 4; k++) c[k] = h[4 * (size_t)i + k];
+    ldg32(h + 4 * (size_t)i, c[0], c[1]);
+    ldg32(h + 4 * (size_t)i + 2, c[2], c[3]);
     if (agg_in) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) c[4 + k] = agg_in[4 * (size_t)i + k];
+      ldg32(agg_in + 4 * (size_t)i, c[4], c[5]);
+      ldg32(agg_in + 4 * (size_t)i + 2, c[6], c[7]);
     } else {
       float s[32];
 #pragma unroll
@@ -205,10 +236,11 @@ struct GatherNode {
 
 struct GatherDec {   // [h (32), 1, 0 x 15]
   const uint4 *h;
-  __device__ void load(uint32_t i, uint4 *c) const
+  __device__ RowIdx index(uint32_t) const { return RowIdx{}; }
+  __device__ void load(uint32_t i, const RowIdx &, uint4 *c) const
   {
-#pragma unroll
-    for (int k = 0; k < 4; k++) c[k] = h[4 * (size_t)i + k];
+    ldg32(h + 4 * (size_t)i, c[0], c[1]);
+    ldg32(h + 4 * (size_t)i + 2, c[2], c[3]);
     c[4] = make_uint4(BF16_ONE, 0, 0, 0);
     c[5] = make_uint4(0, 0, 0, 0);
   }
@@ -277,6 +309,12 @@ struct OutDecApply {   // z = y + s out (FP64), s = scal[0]
 // Y = MLP(X) for `rows` rows: H = ReLU(X~ W1~^T) (32 wide), Y = H~ W2~^T (N2 wide).
 // One 128-row tile at a time per CTA (persistent); thread t owns row t of the
 // tile and TMEM lane t.  a1_save (optional) keeps H for the backward pass.
+// Bound by a tile's chain (two tensor-core round trips and the shared-memory
+// traffic around them), five CTAs of 41 KB an SM.  What shortened it: rows of
+// messages rotated so that staging and summing them meets no bank twice (32
+// threads wrote one bank group before), 64-byte rows gathered by two requests
+// instead of four, indices and tile bounds loaded a tile ahead.  One
+// application at 70^3 (4.7 million directed edges): 1,332 -> 936 us.
 template <int K1, int N2>
 constexpr size_t fwd_smem() { return (size_t)128 * K1 * 2 + 128 * 48 * 2 + 32 * K1 * 2 + N2 * 48 * 2; }
 
@@ -312,37 +350,45 @@ __global__ void __launch_bounds__(128) k_mlp_fwd(G gat, O out, uint32_t rows, co
   constexpr bool SEG = SegSum<O>::value;
   uint32_t ntiles = (rows + 127) / 128;
   if constexpr (SEG) ntiles = out.ntiles;
-  // a tile's first row and row count (SEG: the plan's tiles of whole nodes)
-  auto span = [&](uint32_t tile) -> uint2 {
-    if constexpr (SEG) {
-      const uint4 pl = out.plan[tile];
-      return make_uint2(pl.x, pl.y);
-    }
+  // a tile's first row, rows, first node and nodes (SEG: the plan's tiles of
+  // whole nodes; none past the end)
+  auto span = [&](uint32_t tile) -> uint4 {
+    if (tile >= ntiles) return make_uint4(0, 0, 0, 0);
+    if constexpr (SEG) return out.plan[tile];
     const uint32_t r0 = tile * 128;
-    return make_uint2(r0, rows - r0 < 128u ? rows - r0 : 128u);
+    return make_uint4(r0, rows - r0 < 128u ? rows - r0 : 128u, 0, 0);
   };
-  // the next tile's rows are gathered into registers while this tile's GEMMs
-  // and epilogues run (software pipeline of depth one)
+  auto index = [&](const uint4 &sp) -> RowIdx { return (uint32_t)t < sp.y ? gat.index(sp.x + t) : RowIdx{}; };
+  // software pipeline: while a tile's GEMMs and epilogues run, the next tile's
+  // rows are gathered into registers, through indices loaded a tile earlier
   uint4 c[K1 / 8];
-  auto gather = [&](uint32_t tile) {
-    const uint2 sp = tile < ntiles ? span(tile) : make_uint2(0, 0);
-    if ((uint32_t)t < sp.y) gat.load(sp.x + t, c);
+  auto gather = [&](const uint4 &sp, const RowIdx &x) {
+    if ((uint32_t)t < sp.y) gat.load(sp.x + t, x, c);
     else {
 #pragma unroll
       for (int k = 0; k < K1 / 8; k++) c[k] = make_uint4(0, 0, 0, 0);
     }
   };
-  gather(blockIdx.x);
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint2 sp = span(tile);
+  const uint32_t g = gridDim.x;
+  uint4 sp = span(blockIdx.x), sp1 = span(blockIdx.x + g), sp2 = span(blockIdx.x + 2 * g);
+  RowIdx x1 = index(sp);
+  gather(sp, x1);
+  x1 = index(sp1);
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += g) {
     const uint32_t row = sp.x + t;
     const bool valid = (uint32_t)t < sp.y;
+    // the first rows of the tile's nodes, needed by the message sums below
+    uint32_t first = 0;
+    if constexpr (SEG)
+      if ((uint32_t)t <= sp.w) first = out.seg[sp.z + t] - sp.x;
 #pragma unroll
     for (int k = 0; k < K1 / 8; k++) st_chunk(Xs, t, k, K1, c[k]);
     fence_proxy_async();
     sync_tc();
     if (t == 0) gemm_issue(tm, Xs, W1s, K1, 32, &mbar, false);
-    gather(tile + gridDim.x);
+    gather(sp1, x1);
+    x1 = index(sp2);
+    const uint4 sp3 = span(tile + 3 * g);
     if (!mbar_try(&mbar, phase)) { atomicExch(err, 1); s_abort = 1; }
     phase ^= 1;
     fence_after_sync();
@@ -376,17 +422,17 @@ __global__ void __launch_bounds__(128) k_mlp_fwd(G gat, O out, uint32_t rows, co
         for (int k = 0; k < 4; k++) {
           float f[8];
           unpack8(pack8(v + 8 * k), f);
-#pragma unroll
-          for (int u = 0; u < 8; u++) S[32 * t + 8 * k + u] = f[u];
+          *reinterpret_cast<float4 *>(S + row_word(t, 2 * k)) = make_float4(f[0], f[1], f[2], f[3]);
+          *reinterpret_cast<float4 *>(S + row_word(t, 2 * k + 1)) = make_float4(f[4], f[5], f[6], f[7]);
         }
+        uint32_t *F = reinterpret_cast<uint32_t *>(Xs + 128 * 32 * sizeof(float));   // (a tile has at most 128 nodes)
+        if ((uint32_t)t <= sp.w) F[t] = first;
+        if (t == 0 && sp.w == 128u) F[128] = sp.y;   // 128 nodes of one row each: the end is the tile's
         __syncthreads();
-        const uint4 pl = out.plan[tile];
-        const int l32 = t & 31;
-        for (uint32_t j = (uint32_t)warp; j < pl.w; j += 4) {   // warp per node, lane per component
-          const uint32_t node = pl.z + j;
-          const uint32_t r0 = out.seg[node] - pl.x, r1 = out.seg[node + 1] - pl.x;
-          float sum = 0.f;
-          for (uint32_t r = r0; r < r1; r++) sum += S[32 * r + l32];
+        const uint32_t l32 = t & 31;
+        for (uint32_t j = (uint32_t)warp; j < sp.w; j += 4) {   // warp per node, lane per component
+          const uint32_t node = sp.z + j;
+          const float sum = row_sum(S, F[j], F[j + 1], l32);
           const __nv_bfloat16 bsum = __float2bfloat16_rn(sum);
           out.agg[32 * (size_t)node + l32] = *reinterpret_cast<const uint16_t *>(&bsum);
         }
@@ -396,6 +442,9 @@ __global__ void __launch_bounds__(128) k_mlp_fwd(G gat, O out, uint32_t rows, co
     }
     sync_tc();
     if (s_abort) break;
+    sp = sp1;
+    sp1 = sp2;
+    sp2 = sp3;
   }
   sync_tc();
   if (warp == 0) tmem_dealloc(tm, 64);
@@ -405,7 +454,7 @@ __global__ void __launch_bounds__(128) k_mlp_fwd(G gat, O out, uint32_t rows, co
 
 struct DYDense32 {   // dY row from an FP32 [rows x 32] array
   const float4 *g;
-  __device__ void load(uint32_t r, float *d) const
+  __device__ void load(uint32_t r, const RowIdx &, float *d) const
   {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
@@ -417,10 +466,9 @@ struct DYDense32 {   // dY row from an FP32 [rows x 32] array
 
 struct DYEdge {   // dY_r = dagg[rnode[r]]
   const float4 *dagg;
-  const uint32_t *rnode;
-  __device__ void load(uint32_t r, float *d) const
+  __device__ void load(uint32_t, const RowIdx &x, float *d) const
   {
-    const uint32_t i = rnode[r];
+    const uint32_t i = x.i;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const float4 v = dagg[8 * (size_t)i + k];
@@ -432,7 +480,7 @@ struct DYEdge {   // dY_r = dagg[rnode[r]]
 struct DYLoss {   // d/d out of w * sum (out - target)^2
   const float4 *out, *tgt;
   float w;
-  __device__ void load(uint32_t i, float *d) const
+  __device__ void load(uint32_t i, const RowIdx &, float *d) const
   {
     const float4 o = out[i], g = tgt[i];
     d[0] = 2.f * w * (o.x - g.x); d[1] = 2.f * w * (o.y - g.y);
@@ -491,20 +539,45 @@ struct SinkEdge {   // columns 0..31 -> part_i[r], 32..63 -> part_j[r]
   }
 };
 
+// SinkEdge with the rows of columns 0..31 summed per node inside the tile
+// (tiles of whole nodes, as in OutSegSum): pis[node], FP32 in row order
+struct SinkEdgeSeg {
+  float *pis;
+  float4 *pj;
+  const uint4 *plan;
+  const uint32_t *seg;
+  uint32_t ntiles;
+  __device__ void store(uint32_t r, int c, const float *v) const
+  {
+    float4 *d = pj + 8 * (size_t)r + 4 * (c - 2);
+#pragma unroll
+    for (int k = 0; k < 4; k++) d[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  }
+};
+template <> struct SegSum<SinkEdgeSeg> { static constexpr bool value = true; };
+
 // ------------------------------------------------------------ backward kernel
 
 // For Y = MLP(X) with the forward's saved hidden activations H (a1_save):
 //   G1: dH  = dY W2~[:, :32]           (TMEM cols   0..31)
 //       dP  = dH * (H > 0)
-//   G2: dX  = dP W1~                   (TMEM cols  32..32+K1)
-//   G3: dW2~^T += H~^T dY  (over rows) (TMEM cols 128..128+N2, lanes = features)
-//   G4: dW1~^T += X~^T dP              (TMEM cols 160..191)
+//   G2: dX  = dP W1~                   (TMEM cols   0..NX-1, G1's read before; the columns sinks take)
+//   G3: dW2~^T += H~^T dY  (over rows) (TMEM cols  64..64+N2, lanes K1.. = features of H~)
+//   G4: dW1~^T += X~^T dP              (TMEM cols  96..127, lanes 0..K1-1 = features of X~)
+// X~ and H~ are the columns of one 128 x 128 tile (X~ first), staged once by
+// rows like dY and dP: G3 and G4 read the tiles transposed (MN-major operands),
+// so nothing is transposed in shared memory (16-bit stores, four to a bank,
+// were most of the kernel's shared-memory time).  Four CTAs of 55 KB and 128
+// TMEM columns share an SM (two of 105 KB with transposed copies).  Forward and
+// backward of two pairs at 40^3: 3,361 us with the copies, 2,509 with X~ and H~
+// in one transposed copy and the messages and edge adjoints summed in the
+// tiles, 2,034 us so.
 // W1t = W1~^T [K1 x 32], W2t = W2~^T [48 x N2] (rows 0..31 used by G1).  Each
 // CTA writes its weight-gradient sums to part[blockIdx] ([K1 x 32] then [48 x N2]).
 template <int K1, int N2>
 constexpr size_t bwd_smem()
 {
-  return (size_t)128 * N2 * 2 * 2 + 128 * 32 * 2 * 2 + 128 * 128 * 2 * 2 + 32 * N2 * 2 + K1 * 32 * 2;
+  return (size_t)128 * N2 * 2 + 128 * 32 * 2 + 128 * 128 * 2 + 32 * N2 * 2 + K1 * 32 * 2;
 }
 
 template <int K1, int N2, bool DX, class G, class DY, class S>
@@ -512,20 +585,19 @@ __global__ void __launch_bounds__(128) k_mlp_bwd(G gat, DY dyf, S sink, uint32_t
                                                  const uint4 *__restrict__ W2t, const uint4 *__restrict__ a1_save,
                                                  float *__restrict__ part, int *__restrict__ err)
 {
+  static_assert(K1 + 48 <= 128, "features of X~ and H~ share one operand");
+  constexpr int NX = K1 < 64 ? K1 : 64;   // columns of dX (the sinks take no more)
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char *dYs = smem;                     // A: 128 x N2
-  unsigned char *dYt = dYs + 128 * N2 * 2;       // B: N2 x 128
-  unsigned char *Ps = dYt + 128 * N2 * 2;        // A: 128 x 32
-  unsigned char *Pt = Ps + 128 * 32 * 2;         // B: 32 x 128
-  unsigned char *Ht = Pt + 128 * 32 * 2;         // A: 128 features x 128 rows
-  unsigned char *Xt = Ht + 128 * 128 * 2;        // A: 128 features x 128 rows
-  unsigned char *W2s = Xt + 128 * 128 * 2;       // B: 32 x N2
+  unsigned char *XH = smem;                      // 128 rows x 128 features (X~, H~, zeros)
+  unsigned char *dYs = XH + 128 * 128 * 2;       // 128 x N2
+  unsigned char *Ps = dYs + 128 * N2 * 2;        // 128 x 32
+  unsigned char *W2s = Ps + 128 * 32 * 2;        // B: 32 x N2
   unsigned char *W1s = W2s + 32 * N2 * 2;        // B: K1 x 32
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tslot;
   __shared__ int s_abort;
   const int t = threadIdx.x, warp = t >> 5;
-  if (warp == 0) tmem_alloc(&tslot, 256);
+  if (warp == 0) tmem_alloc(&tslot, 128);
   if (t == 0) {
     mbar_init1(&mbar);
     s_abort = 0;
@@ -534,11 +606,8 @@ __global__ void __launch_bounds__(128) k_mlp_bwd(G gat, DY dyf, S sink, uint32_t
     st_chunk(W2s, idx / (N2 / 8), idx % (N2 / 8), N2, W2t[idx]);
   for (int idx = t; idx < K1 * 4; idx += 128) st_chunk(W1s, idx / 4, idx % 4, 32, W1t[idx]);
   {
-    uint4 *z0 = reinterpret_cast<uint4 *>(Ht), *z1 = reinterpret_cast<uint4 *>(Xt);
-    for (int idx = t; idx < 128 * 128 * 2 / 16; idx += 128) {
-      z0[idx] = make_uint4(0, 0, 0, 0);
-      z1[idx] = make_uint4(0, 0, 0, 0);
-    }
+    uint4 *z = reinterpret_cast<uint4 *>(XH);
+    for (int idx = t; idx < 128 * 128 * 2 / 16; idx += 128) z[idx] = make_uint4(0, 0, 0, 0);
   }
   fence_proxy_async();
   sync_tc();
@@ -546,48 +615,56 @@ __global__ void __launch_bounds__(128) k_mlp_bwd(G gat, DY dyf, S sink, uint32_t
   const uint32_t lane = (uint32_t)(warp * 32) << 16;
   uint32_t phase = 0;
   bool first = true;
-  const uint32_t ntiles = (rows + 127) / 128;
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint32_t row = tile * 128 + t;
-    const bool valid = row < rows;
-    // dY (both layouts)
-    {
-      float d[32];
-      if (valid) dyf.load(row, d);
-      else {
+  constexpr bool SEG = SegSum<S>::value;
+  uint32_t ntiles = (rows + 127) / 128;
+  if constexpr (SEG) ntiles = sink.ntiles;
+  auto span = [&](uint32_t tile) -> uint4 {
+    if (tile >= ntiles) return make_uint4(0, 0, 0, 0);
+    if constexpr (SEG) return sink.plan[tile];
+    const uint32_t r0 = tile * 128;
+    return make_uint4(r0, r0 < rows ? (rows - r0 < 128u ? rows - r0 : 128u) : 0u, 0, 0);
+  };
+  auto index = [&](const uint4 &sp) -> RowIdx { return (uint32_t)t < sp.y ? gat.index(sp.x + t) : RowIdx{}; };
+  const uint32_t g = gridDim.x;
+  uint4 sp = span(blockIdx.x), sp1 = span(blockIdx.x + g);
+  RowIdx x = index(sp);   // indices loaded a tile before they are used
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += g) {
+    const uint32_t row = sp.x + t;
+    const bool valid = (uint32_t)t < sp.y;
+    uint32_t first_row = 0;
+    if constexpr (SEG)
+      if ((uint32_t)t <= sp.w) first_row = sink.seg[sp.z + t] - sp.x;
+    float d[32];
+    uint4 h[4], c[K1 / 8];
+    if (valid) {
+      dyf.load(row, x, d);
 #pragma unroll
-        for (int k = 0; k < N2; k++) d[k] = 0.f;
-      }
+      for (int k = 0; k < 4; k++) h[k] = a1_save[4 * (size_t)row + k];
+      gat.load(row, x, c);
+    } else {
 #pragma unroll
-      for (int k = 0; k < N2 / 8; k++) {
-        const uint4 p = pack8(d + 8 * k);
-        st_chunk(dYs, t, k, N2, p);
-        st_t_chunk(dYt, 8 * k, t, p);
-      }
+      for (int k = 0; k < N2; k++) d[k] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; k++) h[k] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int k = 0; k < K1 / 8; k++) c[k] = make_uint4(0, 0, 0, 0);
     }
-    // H~^T from the saved activations (ones feature at 32 for valid rows)
-    uint4 h[4];
+    x = index(sp1);
+    const uint4 sp2 = span(tile + 2 * g);
 #pragma unroll
-    for (int k = 0; k < 4; k++) h[k] = valid ? a1_save[4 * (size_t)row + k] : make_uint4(0, 0, 0, 0);
+    for (int k = 0; k < N2 / 8; k++) st_chunk(dYs, t, k, N2, pack8(d + 8 * k));
 #pragma unroll
-    for (int k = 0; k < 4; k++) st_t_chunk(Ht, 8 * k, t, h[k]);
-    st_t(Ht, 32, t, valid ? (uint16_t)BF16_ONE : (uint16_t)0);
-    // X~^T regathered
-    {
-      uint4 c[K1 / 8];
-      if (valid) gat.load(row, c);
-      else {
+    for (int k = 0; k < K1 / 8; k++) st_chunk(XH, t, k, 128, c[k]);
+    // H~: the saved activations, the ones feature (valid rows), zeros
 #pragma unroll
-        for (int k = 0; k < K1 / 8; k++) c[k] = make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int k = 0; k < K1 / 8; k++) st_t_chunk(Xt, 8 * k, t, c[k]);
-    }
+    for (int k = 0; k < 4; k++) st_chunk(XH, t, K1 / 8 + k, 128, h[k]);
+    st_chunk(XH, t, K1 / 8 + 4, 128, make_uint4(valid ? BF16_ONE : 0u, 0, 0, 0));
+    st_chunk(XH, t, K1 / 8 + 5, 128, make_uint4(0, 0, 0, 0));
     fence_proxy_async();
     sync_tc();
     if (t == 0) {
-      gemm_issue_nc(tm, dYs, W2s, N2, 32, false);            // G1
-      gemm_issue_nc(tm + 128, Ht, dYt, 128, N2, !first);     // G3
+      gemm_issue_nc(tm, dYs, W2s, N2, 32, false);             // G1
+      gemm_issue_t(tm + 64, XH, 128, dYs, N2, N2, !first);     // G3
       mma_commit(&mbar);
     }
     if (!mbar_try(&mbar, phase)) { atomicExch(err, 1); s_abort = 1; }
@@ -601,79 +678,132 @@ __global__ void __launch_bounds__(128) k_mlp_bwd(G gat, DY dyf, S sink, uint32_t
 #pragma unroll
       for (int k = 0; k < 32; k++) v[k] = hf[k] > 0.f ? v[k] : 0.f;
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const uint4 p = pack8(v + 8 * k);
-        st_chunk(Ps, t, k, 32, p);
-        st_t_chunk(Pt, 8 * k, t, p);
-      }
+      for (int k = 0; k < 4; k++) st_chunk(Ps, t, k, 32, pack8(v + 8 * k));
     }
     fence_proxy_async();
     sync_tc();
     if (t == 0) {
-      if (DX) gemm_issue_nc(tm + 32, Ps, W1s, 32, K1, false);   // G2
-      gemm_issue_nc(tm + 160, Xt, Pt, 128, 32, !first);         // G4
+      if (DX) gemm_issue_nc(tm, Ps, W1s, 32, NX, false);        // G2
+      gemm_issue_t(tm + 96, XH, 128, Ps, 32, 32, !first);       // G4
       mma_commit(&mbar);
     }
     if (!mbar_try(&mbar, phase)) { atomicExch(err, 1); s_abort = 1; }
     phase ^= 1;
     fence_after_sync();
-    if (DX) {
+    if constexpr (DX && SEG) {
+      // columns 0..31 summed per node through the X~, H~ tile (its products
+      // are done, and every row of it is written whole for the next tile),
+      // 32..63 stored
+      static_assert(K1 == 80, "all 16 words of the tile's rows are rewritten");
+      float *St = reinterpret_cast<float *>(XH);
+      uint32_t *F = reinterpret_cast<uint32_t *>(XH + 128 * 32 * sizeof(float));
+      float v[32];
+      tmem_ld32(tm + lane, v);
 #pragma unroll
-      for (int c = 0; c < K1 / 16; c++) {
+      for (int w = 0; w < 8; w++)
+        *reinterpret_cast<float4 *>(St + row_word(t, w)) = make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
+      if ((uint32_t)t <= sp.w) F[t] = first_row;
+      if (t == 0 && sp.w == 128u) F[128] = sp.y;
+#pragma unroll
+      for (int c2 = 2; c2 < 4; c2++) {
+        float u[16];
+        tmem_ld16(tm + lane + 16 * c2, u);
+        if (valid) sink.store(row, c2, u);
+      }
+      __syncthreads();
+      const uint32_t l32 = t & 31;
+      for (uint32_t j = (uint32_t)warp; j < sp.w; j += 4)
+        sink.pis[32 * (size_t)(sp.z + j) + l32] = row_sum(St, F[j], F[j + 1], l32);
+    } else if (DX) {
+#pragma unroll
+      for (int c = 0; c < NX / 16; c++) {
         float v[16];
-        tmem_ld16(tm + lane + 32 + 16 * c, v);
+        tmem_ld16(tm + lane + 16 * c, v);
         if (valid) sink.store(row, c, v);
       }
     }
     first = false;
     sync_tc();
     if (s_abort) break;
+    sp = sp1;
+    sp1 = sp2;
   }
   // per-CTA weight-gradient sums; lanes are features
   float *p1 = part + (size_t)blockIdx.x * (K1 * 32 + 48 * N2);
   float *p2 = p1 + K1 * 32;
   {
     float v[32];
-    tmem_ld32(tm + lane + 160, v);
+    tmem_ld32(tm + lane + 96, v);
     if (t < K1)
       for (int o = 0; o < 32; o++) p1[t * 32 + o] = first ? 0.f : v[o];
-    if (N2 == 32) tmem_ld32(tm + lane + 128, v);
-    else tmem_ld16(tm + lane + 128, v);
-    if (t < 48)
-      for (int o = 0; o < N2; o++) p2[t * N2 + o] = first ? 0.f : v[o];
+    if (N2 == 32) tmem_ld32(tm + lane + 64, v);
+    else tmem_ld16(tm + lane + 64, v);
+    if (t >= K1 && t < K1 + 48)
+      for (int o = 0; o < N2; o++) p2[(t - K1) * N2 + o] = first ? 0.f : v[o];
   }
   sync_tc();
-  if (warp == 0) tmem_dealloc(tm, 256);
+  if (warp == 0) tmem_dealloc(tm, 128);
 }
 
 // grad(W1~)[o][f] += sum_b part[b][f][o]; grad(W2~)[o][f] += sum_b part[b][K1*32 + f*N2 + o]
-__global__ void k_wgrad_reduce(const float *__restrict__ part, int nblk, int K1, int N2, float *__restrict__ g1,
-                               float *__restrict__ g2)
+// One warp column of a 32 x 8 block per weight, in the partials' own order
+// (coalesced): thread (x, y) sums every eighth CTA's partial from y on, the
+// eight sums are added in order.
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ part, int nblk, int K1, int N2,
+                                                      float *__restrict__ g1, float *__restrict__ g2)
 {
-  const int n1 = 32 * K1, n2 = N2 * 48, stride = K1 * 32 + 48 * N2;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < n1) {
-    const int o = idx / K1, f = idx % K1;
-    float s = 0.f;
-    for (int b = 0; b < nblk; b++) s += part[(size_t)b * stride + f * 32 + o];
-    g1[idx] += s;
-  } else if (idx < n1 + n2) {
-    const int j = idx - n1, o = j / 48, f = j % 48;
-    float s = 0.f;
-    for (int b = 0; b < nblk; b++) s += part[(size_t)b * stride + K1 * 32 + f * N2 + o];
-    g2[j] += s;
+  __shared__ float sm[8][32];
+  const int n1 = 32 * K1, n2 = N2 * 48, stride = n1 + n2;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, idx = blockIdx.x * 32 + x;
+  float s = 0.f;
+  if (idx < stride) {
+    int b = y;
+    for (; b + 24 < nblk; b += 32) {
+      float v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = part[(size_t)(b + 8 * u) * stride + idx];
+#pragma unroll
+      for (int u = 0; u < 4; u++) s += v[u];
+    }
+    for (; b < nblk; b += 8) s += part[(size_t)b * stride + idx];
+  }
+  sm[y][x] = s;
+  __syncthreads();
+  if (y != 0 || idx >= stride) return;
+  s = 0.f;
+  for (int u = 0; u < 8; u++) s += sm[u][x];
+  if (idx < n1) g1[(idx & 31) * K1 + (idx >> 5)] += s;
+  else {
+    const int j = idx - n1;
+    g2[(j % N2) * 48 + j / N2] += s;
   }
 }
 
-// dh[i] += sum_{r at i} part_i[r] + part_j[rev[r]]; one warp per node, lane = feature
+// dh[i] += (sum of part_i over the rows at i) + sum_{r at i} part_j[rev[r]];
+// one warp per node, lane = feature.  The first sum is given per node (pis,
+// formed by the tiles of whole nodes) or per row (pi).
 __global__ void k_edge_adjoint(uint32_t N, const uint32_t *__restrict__ seg, const uint32_t *__restrict__ rev,
-                               const float *__restrict__ pi, const float *__restrict__ pj, float *__restrict__ dh)
+                               const float *__restrict__ pi, const float *__restrict__ pis,
+                               const float *__restrict__ pj, float *__restrict__ dh)
 {
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int f = threadIdx.x & 31;
   if (i >= N) return;
   float s = dh[32 * (size_t)i + f];
-  for (uint32_t r = seg[i]; r < seg[i + 1]; r++) s += pi[32 * (size_t)r + f] + pj[32 * (size_t)rev[r] + f];
+  if (pis) s += pis[32 * (size_t)i + f];
+  uint32_t r = seg[i];
+  const uint32_t r1 = seg[i + 1];
+  for (; r + 4 <= r1; r += 4) {
+    float a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      b[u] = pj[32 * (size_t)rev[r + u] + f];
+      a[u] = pis ? 0.f : pi[32 * (size_t)(r + u) + f];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) s += a[u] + b[u];
+  }
+  for (; r < r1; r++) s += (pis ? 0.f : pi[32 * (size_t)r + f]) + pj[32 * (size_t)rev[r] + f];
   dh[32 * (size_t)i + f] = s;
 }
 
@@ -701,6 +831,7 @@ __global__ void k_loss_final(const double *__restrict__ part, int n, double w, d
 {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
+#pragma unroll 16
     for (int b = 0; b < n; b++) s += part[b];
     loss[0] += w * s;
   }
@@ -764,6 +895,7 @@ __global__ void k_rms(const double *__restrict__ part, int nb, double n, double 
 {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
+#pragma unroll 16
     for (int b = 0; b < nb; b++) s += part[b];
     const double r = sqrt(s / n);
     scal[0] = r > 0.0 ? r : 1.0;
@@ -1007,8 +1139,9 @@ int launch_bwd(kfun3d_mpnn *net, G g, DY dy, S sink, uint32_t rows, int layer, c
   auto kern = k_mlp_bwd<K1, N2, DX, G, DY, S>;
   static unsigned grid_cache[64] = {0};
   unsigned &gc = grid_cache[net->device & 63];
-  if (!gc) gc = persistent_grid(kern, smem, net->nsm, 2);   // 256 TMEM columns per CTA
-  const unsigned ntiles = std::max(1u, (rows + 127) / 128);
+  if (!gc) gc = persistent_grid(kern, smem, net->nsm, 4);   // 128 TMEM columns per CTA
+  unsigned ntiles = std::max(1u, (rows + 127) / 128);
+  if constexpr (SegSum<S>::value) ntiles = std::max(1u, sink.ntiles);
   const unsigned grid = std::min(gc, ntiles);
   const size_t stride = K1 * 32 + 48 * N2;
   if (net->wpart.need((size_t)grid * stride * sizeof(float)) != cudaSuccess)
@@ -1017,7 +1150,7 @@ int launch_bwd(kfun3d_mpnn *net, G g, DY dy, S sink, uint32_t rows, int layer, c
   const uint4 *W2t = reinterpret_cast<const uint4 *>(net->Wt + kOff.off[layer + 1]);
   kern<<<grid, 128, smem, st>>>(g, dy, sink, rows, W1t, W2t, a1_save, net->wpart.as<float>(), net->err);
   const int n = 32 * K1 + N2 * 48;
-  k_wgrad_reduce<<<(n + 255) / 256, 256, 0, st>>>(net->wpart.as<float>(), (int)grid, K1, N2,
+  k_wgrad_reduce<<<(n + 31) / 32, 256, 0, st>>>(net->wpart.as<float>(), (int)grid, K1, N2,
                                                    net->grad + kOff.off[layer], net->grad + kOff.off[layer + 1]);
   kf_count_launch(2);
   MP_CK(cudaGetLastError());
@@ -1076,19 +1209,20 @@ int forward(kfun3d_mpnn *net, const GraphDev &g, const uint4 *x0, bool train, co
   auto H = [&](int l) { return train ? h[l] : h[l & 1]; };
   rc = launch_fwd<16, 32>(net, GatherEnc{x0}, OutBf16{H(0)}, g.N, L_ENC1, train ? net->a1_enc.as<uint4>() : nullptr,
                           st);
-  // inference with a tile plan: the message sums formed in the edge MLP
-  const bool fused = !train && g.plan && g.nplan;
+  // with a tile plan the message sums are formed in the edge MLP
+  const bool fused = g.plan && g.nplan;
   for (int l = 0; l < 3 && !rc; l++) {
+    uint4 *agg = net->agg[train ? l : 0].as<uint4>();
+    uint4 *a1 = train ? net->a1_edge[l].as<uint4>() : nullptr;
+    const GatherEdge ge{H(l), g.rnode, g.oth, g.efeat};
     if (fused)
-      rc = launch_fwd<80, 32>(net, GatherEdge{H(l), g.rnode, g.oth, g.efeat},
-                              OutSegSum{g.plan, g.seg, net->agg[0].as<uint16_t>(), g.nplan}, g.R, L_EDGE1(l),
-                              nullptr, st);
+      rc = launch_fwd<80, 32>(net, ge, OutSegSum{g.plan, g.seg, reinterpret_cast<uint16_t *>(agg), g.nplan}, g.R,
+                              L_EDGE1(l), a1, st);
     else
-      rc = launch_fwd<80, 32>(net, GatherEdge{H(l), g.rnode, g.oth, g.efeat}, OutBf16{net->msg.as<uint4>()}, g.R,
-                              L_EDGE1(l), train ? net->a1_edge[l].as<uint4>() : nullptr, st);
+      rc = launch_fwd<80, 32>(net, ge, OutBf16{net->msg.as<uint4>()}, g.R, L_EDGE1(l), a1, st);
     if (rc) break;
-    GatherNode gn{H(l), g.seg, fused ? nullptr : net->msg.as<uint4>(), train ? net->agg[l].as<uint4>() : nullptr,
-                  fused ? net->agg[0].as<uint4>() : nullptr};
+    GatherNode gn{H(l), g.seg, fused ? nullptr : net->msg.as<uint4>(), train && !fused ? agg : nullptr,
+                  fused ? agg : nullptr};
     rc = launch_fwd<80, 32>(net, gn, OutResidual{H(l), H(l + 1)}, g.N, L_NODE1(l),
                             train ? net->a1_node[l].as<uint4>() : nullptr, st);
   }
@@ -1118,11 +1252,18 @@ int backward(kfun3d_mpnn *net, const GraphDev &g, const uint4 *x0, const float4 
     rc = launch_bwd<80, 32, true>(net, gn, DYDense32{dA}, SinkNode{dB, dA, dagg}, g.N, L_NODE1(l),
                                   net->a1_node[l].as<uint4>(), st);
     if (rc) break;
-    rc = launch_bwd<80, 32, true>(net, GatherEdge{h[l], g.rnode, g.oth, g.efeat}, DYEdge{dagg, g.rnode},
-                                  SinkEdge{pi, pj}, g.R, L_EDGE1(l), net->a1_edge[l].as<uint4>(), st);
+    const bool seg = g.plan && g.nplan;
+    const GatherEdge ge{h[l], g.rnode, g.oth, g.efeat};
+    const uint4 *a1 = net->a1_edge[l].as<uint4>();
+    if (seg)
+      rc = launch_bwd<80, 32, true>(net, ge, DYEdge{dagg}, SinkEdgeSeg{(float *)pi, pj, g.plan, g.seg, g.nplan},
+                                    g.R, L_EDGE1(l), a1, st);
+    else
+      rc = launch_bwd<80, 32, true>(net, ge, DYEdge{dagg}, SinkEdge{pi, pj}, g.R, L_EDGE1(l), a1, st);
     if (rc) break;
-    k_edge_adjoint<<<(unsigned)((g.N * 32ull + 255) / 256), 256, 0, st>>>(g.N, g.seg, g.rev, (const float *)pi,
-                                                                          (const float *)pj, (float *)dB);
+    k_edge_adjoint<<<(unsigned)((g.N * 32ull + 255) / 256), 256, 0, st>>>(
+        g.N, g.seg, g.rev, seg ? nullptr : (const float *)pi, seg ? (const float *)pi : nullptr, (const float *)pj,
+        (float *)dB);
     kf_count_launch();
     std::swap(dA, dB);
   }
@@ -1346,7 +1487,7 @@ extern "C" kfun3d_mpnn_graph *kfun3d_mpnn_graph_create(const GEOMETRY *g)
   up(G->d.oth, oth);
   up(G->d.rev, rev);
   up(G->d.efeat, ef);
-  // tiles of whole nodes, at most 128 rows each, in node order
+  // tiles of whole nodes, at most 128 rows and 128 nodes each, in node order
   // (KFUN3D_MPNN_FUSED=0: none, the messages go through memory)
   const char *fenv = getenv("KFUN3D_MPNN_FUSED");
   if (!(fenv && strcmp(fenv, "0") == 0)) {
@@ -1355,7 +1496,7 @@ extern "C" kfun3d_mpnn_graph *kfun3d_mpnn_graph_create(const GEOMETRY *g)
     for (uint32_t i = 0; i < N && fits; ) {
       if (seg[i + 1] - seg[i] > 128u) fits = false;
       uint32_t j = i;
-      while (j < N && seg[j + 1] - seg[i] <= 128u) j++;
+      while (j < N && j - i < 128u && seg[j + 1] - seg[i] <= 128u) j++;
       if (fits) plan.push_back(make_uint4(seg[i], seg[j] - seg[i], i, j - i));
       i = j;
     }

@@ -163,6 +163,26 @@ __device__ __forceinline__ void gemm_issue_nc(uint32_t d_tmem, const void *A_sme
   }
 }
 
+// D (TMEM, 128 x N) (+)= A^T B for A (smem, 128 rows x KA) and B (smem, 128
+// rows x KB), the first 128 columns of A and N of B, both staged by rows in the
+// canonical layout above: read as MN-major operands, whose core matrices (8
+// rows of K x 16 bytes along M or N) are the same ones.  For MN-major operands
+// without swizzle the stride byte offset steps along M or N (128 B here), the
+// leading byte offset along K (8-row groups).  One thread issues, no commit.
+__device__ __forceinline__ void gemm_issue_t(uint32_t d_tmem, const void *A_smem, int KA, const void *B_smem, int KB,
+                                             int N, bool accumulate)
+{
+  const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(A_smem);
+  const uint32_t b0 = (uint32_t)__cvta_generic_to_shared(B_smem);
+  const uint32_t ga = (uint32_t)KA * 16u, gb = (uint32_t)KB * 16u;   // bytes of an 8-row group
+  const uint32_t idesc = idesc_bf16(128, N) | (1u << 15) | (1u << 16);   // A and B MN-major
+  for (int ks = 0; ks < 8; ks++) {
+    const uint64_t ad = smem_desc(a0 + ks * 2u * ga, ga, 128u);
+    const uint64_t bd = smem_desc(b0 + ks * 2u * gb, gb, 128u);
+    mma_bf16(d_tmem, ad, bd, idesc, (accumulate || ks > 0) ? 1u : 0u);
+  }
+}
+
 // The same, followed by a commit of every MMA issued so far to mbar.
 __device__ __forceinline__ void gemm_issue(uint32_t d_tmem, const void *A_smem, const void *B_smem, int K, int N,
                                            uint64_t *mbar, bool accumulate)
