@@ -372,8 +372,11 @@ struct DevMesh {
   double graph_aoa = 0.0;
   bool use_graphs = true;
   double *gs_part = nullptr;      // [64][296] block partial sums, [32][32] lower triangle of the basis' Gram matrix
+  // the count of Gram-Schmidt columns written to the host: on the device, in
+  // the host's pinned memory (beside h_scal), and as the host expects it
+  unsigned *gs_seq_d = nullptr, *h_seq = nullptr, gs_seq = 0;
   unsigned *bar = nullptr;        // grid-barrier words: [0..1] persistent sweep, arrivals of [2..3]
-                                  // Gram-Schmidt; [4] counter of the one-CTA-per-SM sweep
+                                  // Gram-Schmidt, [5] reductions; [4] counter of the one-CTA-per-SM sweep
   uint32_t *lev_ptr_d = nullptr;  // [nlev_l+1 + nlev_u+1] level offsets on the device
   unsigned trsv_pgrid = 0;        // persistent sweep grid
   unsigned trsv_mgrid = 0;        // persistent sweep grid of mode 5 (SMs x trsv_mgrid_per)
@@ -438,9 +441,10 @@ void kfun3d_reset_launch_count_by(unsigned long long n);   // undo counts taken 
 cudaError_t kf_flow_reset(DevMesh &m);
 
 // Jacobian-vector product: the residual and the state it is taken at, and the
-// device scalars (|x|, h).
+// device scalars |x| and sqrt(1 + |q|), h = eps times the latter.
 struct JvArgs {
-  const double *r, *q, *scal;
+  const double *r, *q, *xn, *qn;
+  double eps;
 };
 
 // Kernel families, one set per arithmetic mode (kernels_exact.cu, kernels_fast.cu).

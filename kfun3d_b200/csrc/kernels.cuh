@@ -714,7 +714,8 @@ struct NodePass {
   const uint32_t *bndp, *bnd_ptr, *bnd_ent, *wf_nodes;
   const double *wf_n, *fres;
   const double4 *q;                        // the state, mesh numbering
-  const double *jr, *jw, *jwv, *jq, *jcdt, *jscal;   // JV: r, w, w in visit order or null, q, cdt, (|x|, h)
+  const double *jr, *jw, *jwv, *jq, *jcdt, *jxn, *jqn;   // JV: r, w, w in visit order or null, q, cdt, |x|, h / eps
+  double jeps;
 };
 template <bool JV>
 __global__ void __launch_bounds__(256, 6) k_flux_nodes4(uint32_t N, NodePass a, const double *__restrict__ res,
@@ -769,7 +770,7 @@ __global__ void __launch_bounds__(256, 6) k_flux_nodes4(uint32_t N, NodePass a, 
       }
     }
   if (JV) {
-    const double s = a.jscal[0] / a.jscal[1];
+    const double h = a.jeps * a.jqn[0], s = a.jxn[0] / h;
     acc = (acc - jr + jc * (jw - jq)) * s;
   }
   r[own] = acc;
@@ -2587,15 +2588,15 @@ __global__ void __launch_bounds__(128, MINB)
 
 // ------------------------------------------------------------------ J.v
 
-// src/kernel.c:35-44: y = (y - r + cdt (w - q)) * a, a = |x| / h from the
-// device scalars (scal[ia] = |x|, scal[ia+1] = h).
+// src/kernel.c:35-44: y = (y - r + cdt (w - q)) * a, a = |x| / h, h = eps qn.
 __global__ void k_jv_combine(uint32_t N, double *__restrict__ y, const double *__restrict__ r,
                              const double *__restrict__ w, const double *__restrict__ q,
-                             const double *__restrict__ cdt, const double *__restrict__ scal, int ia)
+                             const double *__restrict__ cdt, const double *__restrict__ xn,
+                             const double *__restrict__ qn, double eps)
 {
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
-  const double a = scal[ia] / scal[ia + 1];
+  const double h = eps * qn[0], a = xn[0] / h;
   const double c = cdt[n];
   const double4 yy = reinterpret_cast<double4 *>(y)[n];
   const double4 rr = reinterpret_cast<const double4 *>(r)[n];
@@ -2726,14 +2727,16 @@ static void residual_or_jv(DevMesh &m, const double *q, double *r, int first_ord
       kf_count_launch();
     }
     NodePass a{m.ord, m.in1_ptr, m.in1_edge, m.eoff, m.bndp, m.bnd_ptr, m.bnd_ent, m.wf_nodes, m.wf_n,
-               (const double *)m.fres, (const double4 *)q, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+               (const double *)m.fres, (const double4 *)q, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0};
     if (jv) {
       a.jr = jv->r;
       a.jw = q;
       a.jwv = m.visit ? (const double *)m.qv : nullptr;
       a.jq = jv->q;
       a.jcdt = m.cdt;
-      a.jscal = jv->scal;
+      a.jxn = jv->xn;
+      a.jqn = jv->qn;
+      a.jeps = jv->eps;
       k_flux_nodes4<true><<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, a, (const double *)m.eres, r);
     } else {
       k_flux_nodes4<false><<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, a, (const double *)m.eres, r);
@@ -2769,7 +2772,7 @@ void residual_jv(DevMesh &m, const double *w, double *y, int first_order, double
 {
   residual_or_jv(m, w, y, first_order, u, v, m.two_pass ? &jv : nullptr);
   if (!m.two_pass) {
-    k_jv_combine<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, y, jv.r, w, jv.q, m.cdt, jv.scal, 0);
+    k_jv_combine<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, y, jv.r, w, jv.q, m.cdt, jv.xn, jv.qn, jv.eps);
     kf_count_launch();
   }
 }

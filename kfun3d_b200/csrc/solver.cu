@@ -6,6 +6,7 @@
 // its operation order; fast mode uses explicit fma() and fixed-shape tree
 // reductions (deterministic run to run).
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -21,7 +22,7 @@ namespace {
 
 constexpr double JV_EPS = 1.490116119384766e-08;   // src/kernel.c:12
 constexpr int RED_BLOCKS = 296;                    // 2 x 148 SMs
-constexpr int S_XN = 40, S_H = 41, S_QN = 42, S_FN = 43, S_T0 = 44, S_CMP = 52;
+constexpr int S_XN = 40, S_QN = 42, S_FN = 43, S_T0 = 44, S_CMP = 52;
 
 inline unsigned nblk(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
@@ -91,9 +92,27 @@ __device__ __forceinline__ double warp_sum(double v)
   return v;
 }
 
+// The last CTA of a grid to arrive (its partial sums written before): true in
+// every thread of that CTA, which then sees all partial sums.  Resets *cnt.
+__device__ __forceinline__ bool last_cta(unsigned *cnt)
+{
+  __shared__ bool last_s;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last_s = atomicAdd(cnt, 1u) == gridDim.x - 1;
+    if (last_s) *cnt = 0;
+  }
+  __syncthreads();
+  if (last_s) __threadfence();
+  return last_s;
+}
+
 // Fast form: fixed grid, fixed tree, so the result is run-to-run identical.
-__global__ void __launch_bounds__(256) k_dot_partial(size_t n, const double *__restrict__ a,
-                                                     const double *__restrict__ b, double *__restrict__ part)
+// The last CTA adds the CTAs' sums.
+__global__ void __launch_bounds__(256) k_dot_fast(size_t n, const double *__restrict__ a,
+                                                  const double *__restrict__ b, double *__restrict__ part,
+                                                  double *__restrict__ out, int op, unsigned *cnt)
 {
   __shared__ double sm[8];
   double s = 0.0;
@@ -114,13 +133,9 @@ __global__ void __launch_bounds__(256) k_dot_partial(size_t n, const double *__r
     v = warp_sum(v);
     if (threadIdx.x == 0) part[blockIdx.x] = v;
   }
-}
-
-__global__ void k_dot_final(const double *__restrict__ part, int np, double *__restrict__ out, int op)
-{
-  __shared__ double sm[8];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) s += part[i];
+  if (!last_cta(cnt)) return;
+  s = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) s += __ldcg(part + i);
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -178,22 +193,6 @@ __device__ __forceinline__ double grid_total(const double *part, int np, double 
 // 120^3 426 / 342 us (2.2 GB, 6.4 TB/s).
 constexpr int GS_BLOCKS = 296;   // 2 x 148 SMs
 constexpr int GS_GROUP = 8;      // basis vectors a pass over w takes at once
-
-// The last CTA of a grid to arrive (its partial sums written before): true in
-// every thread of that CTA, which then sees all partial sums.  Resets *cnt.
-__device__ __forceinline__ bool last_cta(unsigned *cnt)
-{
-  __shared__ bool last_s;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    last_s = atomicAdd(cnt, 1u) == gridDim.x - 1;
-    if (last_s) *cnt = 0;
-  }
-  __syncthreads();
-  if (last_s) __threadfence();
-  return last_s;
-}
 
 // part: [2 (k + 1)][GS_BLOCKS] partial sums (w, then V_k, against each vector);
 // L: [KF_NBASIS][32], row v = V_v . V_j for j < v
@@ -265,11 +264,16 @@ __global__ void __launch_bounds__(256, 2) k_gs_dots(size_t n, const double *__re
   }
 }
 
-// w -= sum_v h[v] V[v] (in that order) and h[k+1] = |w|.  Elements from the
-// last to the first: those k_gs_dots read last may still be in L2.
+// w -= sum_v h[v] V[v] (in that order) and h[k+1] = |w|.  The last CTA also
+// writes the column to the host's pinned memory and then counts it in
+// host_seq, so that the host reads it while the vector is still being scaled
+// (a copy node and a stream synchronisation an iteration before: 25^3 167 ->
+// 153 us an iteration, 40^3 236 -> 215).  Elements from the last to the first:
+// those k_gs_dots read last may still be in L2.
 __global__ void __launch_bounds__(256, 3) k_gs_update(size_t n, double *__restrict__ V, int k,
                                                       double *__restrict__ h, double *__restrict__ part,
-                                                      unsigned *cnt)
+                                                      unsigned *cnt, double *host_h, unsigned *seq,
+                                                      volatile unsigned *host_seq)
 {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ double sm[40];
@@ -307,7 +311,18 @@ __global__ void __launch_bounds__(256, 3) k_gs_update(size_t n, double *__restri
   if (threadIdx.x == 0) part[blockIdx.x] = bs;
   if (!last_cta(cnt)) return;
   const double t = grid_total(part, gridDim.x, sm);
-  if (threadIdx.x == 0) h[k + 1] = sqrt(t);
+  if (threadIdx.x <= k) host_h[threadIdx.x] = hs[threadIdx.x];
+  if (threadIdx.x == 0) {
+    h[k + 1] = sqrt(t);
+    host_h[k + 1] = sqrt(t);
+  }
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned s = *seq + 1;
+    *seq = s;
+    *host_seq = s;
+  }
 }
 
 // w /= |w|
@@ -402,11 +417,6 @@ __global__ void k_jv_shift_visit(uint32_t N, const uint32_t *__restrict__ rowof,
   o.w = fast ? fma(a, xx.w, qq.w) : a * xx.w + qq.w;
   reinterpret_cast<double4 *>(w)[i] = o;
   qv[rowof[i]] = o;
-}
-
-__global__ void k_set_h(double *scal)
-{
-  scal[S_H] = JV_EPS * scal[S_QN];
 }
 
 // src/forces.c:8-120 in the reference's order: per colour an OpenMP
@@ -555,9 +565,8 @@ void dev_reduce(DevMesh &m, const double *a, const double *b, double *out, int o
 {
   const size_t n = 4 * (size_t)m.N;
   if (fast) {
-    k_dot_partial<<<RED_BLOCKS, 256, 0, m.stream>>>(n, a, b, m.red);
-    k_dot_final<<<1, 256, 0, m.stream>>>(m.red, RED_BLOCKS, out, op);
-    kf_count_launch(2);
+    k_dot_fast<<<RED_BLOCKS, 256, 0, m.stream>>>(n, a, b, m.red, out, op, m.bar + 5);
+    kf_count_launch();
   } else {
     k_dot_seq<<<1, 256, 0, m.stream>>>(n, a, b, out, op);
     kf_count_launch();
@@ -585,7 +594,6 @@ void dev_jacvec(DevMesh &m, const Ops &o, const double *x, double *y)
 {
   const size_t n = 4 * (size_t)m.N;
   dev_reduce(m, x, x, m.scal + S_XN, 1, o.fast);
-  k_set_h<<<1, 1, 0, m.stream>>>(m.scal);
   if (m.visit) {
     // the shifted state and its visit-order copy in one pass
     k_jv_shift_visit<<<nblk(m.N, 256), 256, 0, m.stream>>>(m.N, m.rowof, m.scal, x, m.q, m.w, m.qv, o.fast);
@@ -593,12 +601,12 @@ void dev_jacvec(DevMesh &m, const Ops &o, const double *x, double *y)
   } else {
     k_jv_shift<<<nblk(n, 256), 256, 0, m.stream>>>(n, m.scal, x, m.q, m.w, o.fast);
   }
-  kf_count_launch(2);
+  kf_count_launch();
   double u, v;
   kfun3d_get_freestream(&u, &v);
   const int fo = kf_first_order();
   if (!fo) o.gradient(m, m.w);
-  o.residual_jv(m, m.w, y, fo, u, v, JvArgs{m.r, m.q, m.scal + S_XN});
+  o.residual_jv(m, m.w, y, fo, u, v, JvArgs{m.r, m.q, m.scal + S_XN, m.scal + S_QN, JV_EPS});
 }
 
 void dev_axpy(DevMesh &m, double a, const double *x, double *y, bool fast)
@@ -651,7 +659,9 @@ void gram_schmidt(DevMesh &m, int k)
   const size_t n = 4 * (size_t)m.N;
   const unsigned grid = std::min((unsigned)GS_BLOCKS, std::max(1u, nblk(n / 2, 256)));
   k_gs_dots<<<grid, 256, 0, m.stream>>>(n, m.V, k, m.scal, m.gs_part, m.gs_part + 64 * GS_BLOCKS, m.bar + 2);
-  launch_dependent(k_gs_update, grid, m.stream, n, m.V, k, m.scal, m.gs_part, m.bar + 3);
+  launch_dependent(k_gs_update, grid, m.stream, n, m.V, k, m.scal, m.gs_part, m.bar + 3, m.h_scal, m.gs_seq_d,
+                   (volatile unsigned *)m.h_seq);
+  m.gs_seq++;
   launch_dependent(k_gs_scale, std::max(1u, nblk(n / 2, 256)), m.stream, n, m.V, k, (const double *)m.scal);
   kf_count_launch(3);
 }
@@ -691,7 +701,27 @@ void arnoldi_step(DevMesh &m, const Ops &o, int k, int prec)
   dev_normalize(m, Vb(m, k + 1), m.scal + k + 1, o.fast);
 }
 
-// Fast mode: the Arnoldi step and the read-back of its Hessenberg column as
+// Waits for the Hessenberg column of the last gram_schmidt in h_scal[0..k+1]:
+// it is there when the kernel's count reaches the host's.  The stream's own
+// state ends the wait when the kernel did not get that far.
+void wait_column(DevMesh &m, int k)
+{
+  volatile unsigned *seq = m.h_seq;
+  for (unsigned spin = 1; *seq != m.gs_seq; spin++) {
+    if (spin % 1024) continue;
+    const cudaError_t e = cudaStreamQuery(m.stream);
+    if (e == cudaErrorNotReady) continue;
+    CK(e);
+    if (*seq != m.gs_seq) {   // idle without it: read back what there is, and count from here
+      m.gs_seq = *seq;
+      fetch(m, 0, k + 2);
+    }
+    break;
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+}
+
+// Fast mode: the Arnoldi step (its Hessenberg column written to the host) as
 // one CUDA graph per (precision, first order, k), captured on first use.
 void arnoldi_step_graph(DevMesh &m, const Ops &o, int k, int prec)
 {
@@ -712,8 +742,9 @@ void arnoldi_step_graph(DevMesh &m, const Ops &o, int k, int prec)
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(m.stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
+      const unsigned seq = m.gs_seq;
       arnoldi_step(m, o, k, prec);
-      cudaMemcpyAsync(m.h_scal, m.scal, (k + 2) * sizeof(double), cudaMemcpyDeviceToHost, m.stream);
+      m.gs_seq = seq;
       e = cudaStreamEndCapture(m.stream, &graph);
     }
     const unsigned nodes = (unsigned)(kfun3d_launch_count() - before);
@@ -732,8 +763,9 @@ void arnoldi_step_graph(DevMesh &m, const Ops &o, int k, int prec)
     m.arnoldi_nodes[prec][fo][k] = nodes;
   }
   CK(cudaGraphLaunch(ge, m.stream));
+  m.gs_seq++;
   kf_count_launch(m.arnoldi_nodes[prec][fo][k]);
-  CK(cudaStreamSynchronize(m.stream));
+  wait_column(m, k);
 }
 
 // Device status words: [0] pivot failure in ILU(0), [1] a bounded wait gave up.
@@ -1397,9 +1429,14 @@ struct Scratch {
   double *buf = nullptr;
   size_t cap = 0;
   cudaStream_t stream = nullptr;
+  unsigned *cnt = nullptr;   // CTAs of a reduction that have arrived
   double *ensure(size_t n)
   {
-    if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    if (!stream) {
+      CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+      CK(cudaMalloc(&cnt, sizeof(unsigned)));
+      CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned), stream));
+    }
     if (n > cap) {
       if (buf) cudaFree(buf);
       cap = std::max(n, (size_t)1 << 16);
@@ -1417,9 +1454,8 @@ double blas_reduce(size_t sz, const double *hv, int op)
   double *red = d + 3 * g_scr.cap, out = 0.0;
   CK(cudaMemcpyAsync(d, hv, sz * sizeof(double), cudaMemcpyHostToDevice, s));
   if (kf_mode() == KFUN3D_MODE_FAST) {
-    k_dot_partial<<<RED_BLOCKS, 256, 0, s>>>(sz, d, d, red + 8);
-    k_dot_final<<<1, 256, 0, s>>>(red + 8, RED_BLOCKS, red, op);
-    kf_count_launch(2);
+    k_dot_fast<<<RED_BLOCKS, 256, 0, s>>>(sz, d, d, red + 8, red, op, g_scr.cnt);
+    kf_count_launch();
   } else {
     k_dot_seq<<<1, 256, 0, s>>>(sz, d, d, red, op);
     kf_count_launch();
@@ -1470,9 +1506,8 @@ extern "C" double Normalize(const size_t sz, double *x)
   double *red = d + 3 * g_scr.cap, nrm = 0.0;
   CK(cudaMemcpyAsync(d, x, sz * sizeof(double), cudaMemcpyHostToDevice, s));
   if (kf_mode() == KFUN3D_MODE_FAST) {
-    k_dot_partial<<<RED_BLOCKS, 256, 0, s>>>(sz, d, d, red + 8);
-    k_dot_final<<<1, 256, 0, s>>>(red + 8, RED_BLOCKS, red, 1);
-    kf_count_launch(2);
+    k_dot_fast<<<RED_BLOCKS, 256, 0, s>>>(sz, d, d, red + 8, red, 1, g_scr.cnt);
+    kf_count_launch();
   } else {
     k_dot_seq<<<1, 256, 0, s>>>(sz, d, d, red, 1);
     kf_count_launch();
