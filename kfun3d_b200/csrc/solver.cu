@@ -35,6 +35,31 @@ inline unsigned nblk(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t);
 // (4,000 elements): 1,281 us with one warp that passed the products around by
 // shuffles, 402 us so (their chains alone: 284 us).
 constexpr int SEQ_TILE = 896;   // 4 products for each of the 224 threads
+// s plus the tile's first cnt products, one after the other; eight
+// shared-memory loads ahead of the additions that use them
+__device__ __forceinline__ double add_in_order(double s, const double *tile, int cnt)
+{
+  const double2 *p = reinterpret_cast<const double2 *>(tile);
+  double2 cur[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) cur[q] = p[q];
+  int i = 0;
+  for (; i + 16 <= cnt; i += 16) {
+    const int nx = i + 32 <= SEQ_TILE ? i / 2 + 8 : 0;
+    double2 nxt[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) nxt[q] = p[nx + q];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      s += cur[q].x;
+      s += cur[q].y;
+      cur[q] = nxt[q];
+    }
+  }
+  for (; i < cnt; i++) s += tile[i];
+  return s;
+}
+
 __global__ void __launch_bounds__(256) k_dot_seq(size_t n, const double *__restrict__ a, const double *__restrict__ b,
                                                  double *__restrict__ out, int op)
 {
@@ -55,27 +80,8 @@ __global__ void __launch_bounds__(256) k_dot_seq(size_t n, const double *__restr
         for (int q = 0; q < 4; q++) tile[t & 1][threadIdx.x - 32 + 224 * q] = u[q] * v[q];
       }
     } else if (threadIdx.x == 0 && t > 0) {
-      // eight shared-memory loads ahead of the additions that use them
-      const double2 *p = reinterpret_cast<const double2 *>(tile[(t - 1) & 1]);
       const size_t left = n - (t - 1) * SEQ_TILE;
-      const int cnt = left < SEQ_TILE ? (int)left : SEQ_TILE;
-      double2 cur[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) cur[q] = p[q];
-      int i = 0;
-      for (; i + 16 <= cnt; i += 16) {
-        const int nx = i + 32 <= SEQ_TILE ? i / 2 + 8 : 0;
-        double2 nxt[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) nxt[q] = p[nx + q];
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          s += cur[q].x;
-          s += cur[q].y;
-          cur[q] = nxt[q];
-        }
-      }
-      for (; i < cnt; i++) s += reinterpret_cast<const double *>(p)[i];
+      s = add_in_order(s, tile[(t - 1) & 1], left < SEQ_TILE ? (int)left : SEQ_TILE);
     }
     __syncthreads();
   }
@@ -337,14 +343,58 @@ __global__ void __launch_bounds__(256) k_gs_scale(size_t n, double *__restrict__
   w[i] = make_double2(a.x * sc, a.y * sc);
 }
 
-// y = (mult * coef[0]) * x + y with the coefficient on the device
-__global__ void k_axpy_dev(size_t n, const double *__restrict__ coef, double mult, const double *__restrict__ x,
-                           double *__restrict__ y, int fast)
+// Exact-mode modified Gram-Schmidt of V[k+1] against V[0..k] and its
+// normalisation (src/kernel.c:129-141) in one launch of one CTA: every dot
+// product's additions form one chain in index order, and the chains follow one
+// another, so one thread adds and the others apply the projection before it
+// and form the products a tile ahead.  At Arnoldi index 15 on the 10^3 mesh the
+// chains alone take 284 us; a launch for each dot product and each projection
+// took 402 us, this one takes 319.
+__global__ void __launch_bounds__(256) k_mgs_seq(size_t n, double *V, int k, double *__restrict__ h)
 {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double a = mult * coef[0];
-  y[i] = fast ? fma(a, x[i], y[i]) : a * x[i] + y[i];
+  __shared__ __align__(16) double tile[2][SEQ_TILE];
+  __shared__ double hs;
+  const size_t nt = (n + SEQ_TILE - 1) / SEQ_TILE;
+  double *w = V + (size_t)(k + 1) * n;
+  for (int v = 0; v <= k + 1; v++) {
+    const double *prev = v > 0 ? V + (size_t)(v - 1) * n : nullptr, *cur = v <= k ? V + (size_t)v * n : nullptr;
+    const double a = v > 0 ? -1.0 * hs : 0.0;
+    double s = 0.0;
+    for (size_t t = 0; t <= nt; t++) {
+      if (threadIdx.x >= 32) {
+        if (t < nt) {
+          double x[4], y[4], z[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const size_t g = t * SEQ_TILE + (threadIdx.x - 32) + 224 * q;
+            x[q] = g < n ? w[g] : 0.0;
+            y[q] = prev && g < n ? prev[g] : 0.0;
+            z[q] = cur && g < n ? cur[g] : 0.0;
+          }
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const size_t g = t * SEQ_TILE + (threadIdx.x - 32) + 224 * q;
+            if (prev) {
+              x[q] = a * y[q] + x[q];
+              if (g < n) w[g] = x[q];
+            }
+            tile[t & 1][threadIdx.x - 32 + 224 * q] = x[q] * (cur ? z[q] : x[q]);
+          }
+        }
+      } else if (threadIdx.x == 0 && t > 0) {
+        const size_t left = n - (t - 1) * SEQ_TILE;
+        s = add_in_order(s, tile[(t - 1) & 1], left < SEQ_TILE ? (int)left : SEQ_TILE);
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      hs = v <= k ? s : sqrt(s);
+      h[v] = hs;
+    }
+    __syncthreads();
+  }
+  const double nrm = hs;
+  for (size_t i = threadIdx.x; i < n; i += blockDim.x) w[i] *= (1.0 / nrm);
 }
 
 // y = a x + y (src/utils.c:69-87)
@@ -666,39 +716,24 @@ void gram_schmidt(DevMesh &m, int k)
   kf_count_launch(3);
 }
 
-// One Arnoldi step k (src/kernel.c:123-141): V[k+1] = M^-1 J V[k],
-// modified Gram-Schmidt against V[0..k], normalised; h in scal[0..k+1].
 // Modified Gram-Schmidt of V[k+1] against V[0..k], normalised; h in scal[0..k+1].
 void orthogonalize(DevMesh &m, const Ops &o, int k)
 {
-  const size_t n = 4 * (size_t)m.N;
-  if (o.fast && (n % 2) == 0) {
+  if (o.fast) {
     gram_schmidt(m, k);
     return;
   }
-  for (int v = 0; v <= k; v++) {
-    dev_reduce(m, Vb(m, k + 1), Vb(m, v), m.scal + v, 0, o.fast);
-    k_axpy_dev<<<nblk(n, 256), 256, 0, m.stream>>>(n, m.scal + v, -1.0, Vb(m, v), Vb(m, k + 1), o.fast);
-    kf_count_launch();
-  }
-  dev_normalize(m, Vb(m, k + 1), m.scal + k + 1, o.fast);
+  k_mgs_seq<<<1, 256, 0, m.stream>>>(4 * (size_t)m.N, m.V, k, m.scal);
+  kf_count_launch();
 }
 
+// One Arnoldi step k (src/kernel.c:123-141): V[k+1] = M^-1 J V[k],
+// orthogonalised and normalised; h in scal[0..k+1].
 void arnoldi_step(DevMesh &m, const Ops &o, int k, int prec)
 {
-  const size_t n = 4 * (size_t)m.N;
   dev_jacvec(m, o, Vb(m, k), m.t);
   o.sptrsv(m, m.t, Vb(m, k + 1), prec);
-  if (o.fast && (n % 2) == 0) {
-    gram_schmidt(m, k);
-    return;
-  }
-  for (int v = 0; v <= k; v++) {
-    dev_reduce(m, Vb(m, k + 1), Vb(m, v), m.scal + v, 0, o.fast);
-    k_axpy_dev<<<nblk(n, 256), 256, 0, m.stream>>>(n, m.scal + v, -1.0, Vb(m, v), Vb(m, k + 1), o.fast);
-    kf_count_launch();
-  }
-  dev_normalize(m, Vb(m, k + 1), m.scal + k + 1, o.fast);
+  orthogonalize(m, o, k);
 }
 
 // Waits for the Hessenberg column of the last gram_schmidt in h_scal[0..k+1]:
@@ -1581,18 +1616,7 @@ extern "C" double kfun3d_time_kernel(GEOMETRY *g, int which, int reps)
       case 3: o.fill(*m, m->q, u, v, prec); o.ilu(*m, prec); break;
       case 4: o.sptrsv(*m, m->r, m->t, prec); break;
       case 5: arnoldi_step(*m, o, 15, prec); break;
-      case 6:
-        if (o.fast) {
-          gram_schmidt(*m, 15);
-          break;
-        }
-        for (int vv = 0; vv <= 15; vv++) {
-          dev_reduce(*m, Vb(*m, 16), Vb(*m, vv), m->scal + vv, 0, o.fast);
-          k_axpy_dev<<<nblk(n, 256), 256, 0, m->stream>>>(n, m->scal + vv, -1.0, Vb(*m, vv), Vb(*m, 16), o.fast);
-          kf_count_launch();
-        }
-        dev_normalize(*m, Vb(*m, 16), m->scal + 16, o.fast);
-        break;
+      case 6: orthogonalize(*m, o, 15); break;
       case 7: o.gradient(*m, m->q); break;
       case 8: o.residual(*m, m->q, m->r, kf_first_order(), u, v); break;
       default: break;
