@@ -441,7 +441,7 @@ static void release_device(MatrixHandle *h)
                   m->diag, m->tblk, m->lpos, m->last_lower, m->lev_l, m->lev_u, m->A, m->lslot, m->dinv,
                   m->Af, m->dinvf, m->q, m->r, m->gx, m->gy, m->gz, m->cdt, m->w, m->t, m->x, m->rhs, m->V,
                   m->red, m->scal, m->forces, m->dscr, m->status, m->flags, m->ticket, m->gs_part, m->gs_seq_d, m->lsq_coef,
-                  m->qv, m->xyzv, m->gxv, m->gyv, m->gzv, m->inc_othv, m->n0v, m->n1v, m->inc_geo, m->desc_l, m->desc_u, m->eoff, m->n1, m->in1_ptr, m->in1_edge, m->eres, m->n0s, m->pair_ptr, m->pairs, m->lev_ptr_d, m->bar, m->Z, m->qold, m->fy, m->fx, m->pscr, m->ord, m->rowof, m->egeo_s, m->sub_part};
+                  m->qv, m->xyzv, m->rec, m->inc_othv, m->n0v, m->n1v, m->inc_geo, m->desc_l, m->desc_u, m->eoff, m->n1, m->in1_ptr, m->in1_edge, m->eres, m->n0s, m->pair_ptr, m->pairs, m->lev_ptr_d, m->bar, m->Z, m->qold, m->fy, m->fx, m->pscr, m->ord, m->rowof, m->egeo_s, m->sub_part};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (m->h_scal) cudaFreeHost(m->h_scal);
@@ -777,6 +777,17 @@ DevMesh *kf_device(const GEOMETRY *g)
     if (genv && strcmp(genv, "plain") == 0) tma = false;
     if (genv && strcmp(genv, "tma") == 0) tma = smem <= 200 * 1024;
     m->grad_smem = tma ? (unsigned)smem : 0;
+    if (m->two_pass) {
+      // the records' gradient: the widest 64-node range staged, up to 100 KB
+      size_t widest = 0;
+      for (uint32_t nb = 0; nb < N; nb += 64) {
+        const uint32_t ne = std::min<uint32_t>(nb + 64, N);
+        widest = std::max<size_t>(widest, ((ptr[ne] + 3u) & ~3u) - (ptr[nb] & ~3u));
+      }
+      const bool plain = genv && strcmp(genv, "plain") == 0;
+      m->rec_smem = 28 * widest <= 100 * 1024 && !plain ? (unsigned)(28 * widest) : 0;
+      KF_CUDA(cudaMalloc(&m->rec, 4 * (size_t)std::max(N, 1u) * sizeof(double4)));
+    }
   }
   // wall faces (colour order) with normals -(1/6) a x b (src/flux.c:485-508)
   {

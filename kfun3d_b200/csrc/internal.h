@@ -293,18 +293,19 @@ struct DevMesh {
   double *inc_w = nullptr;        // [3][wstride] least-squares terms seen from the node
   uint32_t wstride = 0;           // 2E rounded up to a multiple of 4 (16-byte aligned rows)
   unsigned grad_smem = 0;         // dynamic shared memory of k_gradient_tma (0: not used)
+  unsigned rec_smem = 0;          // that of k_gradient_rec (0: not staged)
+  double4 *rec = nullptr;         // [4N] per node and component {q, gx, gy, gz}: state and gradients of the two-pass residual
   double4 *lsq_coef = nullptr;    // [2N] least-squares coefficients per node, computed on the device
   // host wall time of the set-up, microseconds: the whole device mirror, its
   // block pattern on the device, the spatial ILU(0) order's set (0 until built)
   long setup_us = 0, pattern_us = 0, spatial_us = 0;
   long host_pattern_us = -1;      // the same pattern on the host threads (set by the pattern check)
   bool lsq_match = false;         // the terms recomputed from lsq_coef equal the stored ones bit for bit
-  int grad_lanes = 1;             // lanes per node of the gradient in the mesh's order (1 or 4)
   // visit-order copies for the residual passes on large meshes (spatial_order
   // and two_pass): state, coordinates, gradients, the other end of each
   // incidence and the end points of each stored edge as visit positions
   bool visit = false;
-  double4 *qv = nullptr, *xyzv = nullptr, *gxv = nullptr, *gyv = nullptr, *gzv = nullptr;
+  double4 *qv = nullptr, *xyzv = nullptr;
   uint32_t *inc_othv = nullptr, *n0v = nullptr, *n1v = nullptr;
   double4 *inc_geo = nullptr;     // [2E] edge geometry per incidence (CSR order), for the time step and fill
   // two-pass residual (every edge has n0 < n1); edge arrays in storage

@@ -261,6 +261,11 @@ __device__ __forceinline__ double4 ldg4(const double4 *p)
   return v;
 }
 
+__device__ __forceinline__ void stg4(double4 *p, const double4 &v)
+{
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w) : "memory");
+}
+
 // ------------------------------------------------------------------ TMA bulk staging
 
 // 1-D bulk copies (cp.async.bulk, the TMA engine's untiled path) into shared
@@ -527,59 +532,108 @@ __global__ void __launch_bounds__(128) k_lsq_check(uint32_t N, const uint32_t *_
   if (nbad) atomicAdd(bad, nbad);
 }
 
-// The gradient with four lanes per node, lane r owning state component r:
-// each lane sums its component's three gradient entries over the node's
-// incident edges in edge order (the same additions as one thread doing all
-// four components, so the same result).  A quad of lanes reads one 32-byte
-// state record per edge and shares the index and term loads; a lane keeps 3
-// accumulators instead of 12, so four times as many nodes are in flight.
+// The gradient for the two-pass residual, four lanes per node, lane r owning
+// state component r: each lane sums its component's three gradient entries
+// over the node's incident edges in edge order (the same additions as one
+// thread doing all four components) and writes them with the state as one
+// 32-byte record {q_r, gx_r, gy_r, gz_r}, so that a node's four records are one
+// 128-byte line: what the edge pass reads of an end point in one request.
+// The CTA's incidence range (other ends and least-squares terms, 28 bytes an
+// incidence) is contiguous and comes into shared memory by four bulk copies,
+// widened to 4-entry boundaries (the arrays are padded).  Read from global
+// memory, every quad's loads of them went through L1 on their own: wavefronts
+// of the L1 data path were 69 % busy and what bounded the kernel: 25^3 8.3 -> 6.2
+// us, 70^3 74 -> 49, 120^3 265 -> 209 (890 MB algorithmic: 4.3 TB/s).
+// STAGED false: the range of some CTA exceeds shared memory.
 // ord == nullptr: node data in visit order (row p of the incidence is node p
-// of q and of the outputs).
-__global__ void __launch_bounds__(256, 4) k_gradient4(uint32_t N, const uint32_t *__restrict__ ord,
-                                                      const uint32_t *__restrict__ inc_ptr,
-                                                      const uint32_t *__restrict__ inc_oth,
-                                                      const double *__restrict__ inc_w, uint32_t ninc,
-                                                      const double *__restrict__ q, double *__restrict__ gx,
-                                                      double *__restrict__ gy, double *__restrict__ gz)
+// of q and of the records).
+constexpr uint32_t KF_GRAD_NODES = 64;
+template <bool STAGED>
+__global__ void __launch_bounds__(4 * KF_GRAD_NODES) k_gradient_rec(uint32_t N, const uint32_t *__restrict__ ord,
+                                                                    const uint32_t *__restrict__ inc_ptr,
+                                                                    const uint32_t *__restrict__ inc_oth,
+                                                                    const double *__restrict__ inc_w, uint32_t wstride,
+                                                                    const double *__restrict__ q,
+                                                                    double4 *__restrict__ rec, int *err)
 {
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t p = gid >> 2, r = gid & 3;
-  if (p >= N) return;
-  const uint32_t n = ord ? ord[p] : p;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t mbar;
+  const uint32_t nb = blockIdx.x * KF_GRAD_NODES, ne = min(nb + KF_GRAD_NODES, N);
+  const uint32_t p = nb + (threadIdx.x >> 2), r = threadIdx.x & 3;
+  const uint32_t *oth = inc_oth;
+  const double *w0 = inc_w, *w1 = inc_w + wstride, *w2 = inc_w + 2 * (size_t)wstride;
+  uint32_t k = 0, k1 = 0;
+  if (p < N) {
+    k = inc_ptr[p];
+    k1 = inc_ptr[p + 1];
+  }
+  bool ok = true;
+  if (STAGED) {
+    const uint32_t ka = inc_ptr[nb] & ~3u, kb = (inc_ptr[ne] + 3u) & ~3u, cnt = kb - ka;
+    double *s_w = reinterpret_cast<double *>(smem);
+    uint32_t *s_oth = reinterpret_cast<uint32_t *>(smem + 24 * (size_t)cnt);
+    if (threadIdx.x == 0) {
+      mbar_init(&mbar, 1);
+      mbar_expect_tx(&mbar, cnt * 28u);
+      if (cnt) {
+        bulk_g2s(s_w, w0 + ka, cnt * 8u, &mbar);
+        bulk_g2s(s_w + cnt, w1 + ka, cnt * 8u, &mbar);
+        bulk_g2s(s_w + 2 * (size_t)cnt, w2 + ka, cnt * 8u, &mbar);
+        bulk_g2s(s_oth, inc_oth + ka, cnt * 4u, &mbar);
+      }
+    }
+    __syncthreads();
+    ok = mbar_wait(&mbar, 0, err);
+    oth = s_oth;
+    w0 = s_w;
+    w1 = s_w + cnt;
+    w2 = s_w + 2 * (size_t)cnt;
+    k -= ka;
+    k1 -= ka;
+  }
+  const uint32_t n = p < N ? (ord ? ord[p] : p) : 0u;
+  if (!ok || p >= N) return;
   const double qn = q[4 * (size_t)n + r];
   double ax = 0.0, ay = 0.0, az = 0.0;
-  const uint32_t k1 = inc_ptr[p + 1];
-  uint32_t k = inc_ptr[p];
-  // four incidences' loads in flight, added in edge order
+  // four incidences' gathers in flight, added in edge order
   for (; k + 4 <= k1; k += 4) {
-    double dq[4], w[3][4];
+    double dq[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      dq[u] = q[4 * (size_t)inc_oth[k + u] + r];
-#pragma unroll
-      for (int d = 0; d < 3; d++) w[d][u] = inc_w[d * (size_t)ninc + k + u];
-    }
+    for (int u = 0; u < 4; u++) dq[u] = q[4 * (size_t)oth[k + u] + r];
 #pragma unroll
     for (int u = 0; u < 4; u++) {
       const double d = dq[u] - qn;
-      ax += w[0][u] * d;
-      ay += w[1][u] * d;
-      az += w[2][u] * d;
+      ax += w0[k + u] * d;
+      ay += w1[k + u] * d;
+      az += w2[k + u] * d;
     }
   }
   for (; k < k1; k++) {
-    const double d = q[4 * (size_t)inc_oth[k] + r] - qn;
-    ax += inc_w[k] * d;
-    ay += inc_w[ninc + k] * d;
-    az += inc_w[2 * (size_t)ninc + k] * d;
+    const double d = q[4 * (size_t)oth[k] + r] - qn;
+    ax += w0[k] * d;
+    ay += w1[k] * d;
+    az += w2[k] * d;
   }
-  gx[4 * (size_t)n + r] = ax;
-  gy[4 * (size_t)n + r] = ay;
-  gz[4 * (size_t)n + r] = az;
+  stg4(rec + 4 * (size_t)n + r, make_double4(qn, ax, ay, az));
+}
+
+// The gradients of the records in the mesh's numbering (ord: record p belongs
+// to node ord[p]; null: to node p).
+__global__ void __launch_bounds__(256) k_unpack_gradient(uint32_t N, const uint32_t *__restrict__ ord,
+                                                         const double4 *__restrict__ rec, double *__restrict__ gx,
+                                                         double *__restrict__ gy, double *__restrict__ gz)
+{
+  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x, p = gid >> 2, c = gid & 3;
+  if (p >= N) return;
+  const size_t own = 4 * (size_t)(ord ? ord[p] : p) + c;
+  const double4 v = rec[gid];
+  gx[own] = v.y;
+  gy[own] = v.z;
+  gz[own] = v.w;
 }
 
 // Node data in the visit order of the node-centric passes: dst[p] =
-// src[ord[p]] (gather) and back (scatter).  On large meshes the residual
+// src[ord[p]].  On large meshes the residual
 // passes work on visit-ordered copies of the state, coordinates and
 // gradients, so that a node's neighbours -- close to it in space, hence in
 // the Morton visit order -- are close to it in memory too.
@@ -588,13 +642,6 @@ __global__ void __launch_bounds__(256) k_visit_gather(uint32_t N, const uint32_t
 {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < N) dst[p] = src[ord[p]];
-}
-
-__global__ void __launch_bounds__(256) k_visit_scatter(uint32_t N, const uint32_t *__restrict__ ord,
-                                                       const double4 *__restrict__ src, double4 *__restrict__ dst)
-{
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < N) dst[ord[p]] = src[p];
 }
 
 // ------------------------------------------------------------------ residual
@@ -662,44 +709,102 @@ __global__ void __launch_bounds__(128) k_residual(uint32_t N, const uint32_t *__
 // (fq: the state in the mesh's numbering), which the node pass adds: its long
 // chain of square roots and divisions then runs beside the edges instead of
 // in a launch of its own after them (edges, nodes and boundary at 25^3: 28.5 ->
-// 18.5 us).  End points are read as 256-bit records.  Seven CTAs an SM (72
-// registers): 522 us with the node pass at 120^3, 532 with five, 582 with six.
+// 18.5 us).  End points are read as 256-bit records.
+//
+// Second order: the quad of lanes that holds edges 4 i .. 4 i + 3 reads an end
+// point's four records (k_gradient_rec) in one request of one 128-byte line,
+// lane c its component's state and gradient; it reconstructs component c of
+// all four edges, and a 4 x 4 transpose inside the quad gives each lane its own
+// edge's state.  With a lane reading the state and the gradients of its own
+// edge's ends, each in a request of its own, the L1 data path was 75 % busy and
+// bounded the kernel.  Edges and nodes at 70^3 142 -> 123 us, at 120^3 522 -> 515
+// (there the 384 MB of edge fluxes, written once and read twice, take 173 us at
+// a copy's rate); seven CTAs an SM (at 120^3 six take 550 us, five 581, eight 524
+// with the records loaded in two halves).
+// (not inlined: its registers are not the edges')
+__device__ __noinline__ void farfield_store(double U, double V, const double *fn, const double4 *q, double4 *out)
+{
+  *out = farfield_flux(U, V, fn[0], fn[1], fn[2], *q);
+}
+
+__device__ __forceinline__ void quad_transpose(double *L, int c)
+{
+  double a = (c & 1) ? L[0] : L[1], b = (c & 1) ? L[2] : L[3];
+  a = __shfl_xor_sync(0xffffffffu, a, 1);
+  b = __shfl_xor_sync(0xffffffffu, b, 1);
+  if (c & 1) { L[0] = a; L[2] = b; }
+  else { L[1] = a; L[3] = b; }
+  a = (c & 2) ? L[0] : L[2];
+  b = (c & 2) ? L[1] : L[3];
+  a = __shfl_xor_sync(0xffffffffu, a, 2);
+  b = __shfl_xor_sync(0xffffffffu, b, 2);
+  if (c & 2) { L[0] = a; L[1] = b; }
+  else { L[2] = a; L[3] = b; }
+}
+
 template <bool FIRST_ORDER>
 __global__ void __launch_bounds__(128, 7) k_flux_edges(uint32_t E, const uint32_t *__restrict__ n0,
-                                                    const uint32_t *__restrict__ n1,
-                                                    const double4 *__restrict__ egeo,
-                                                    const double4 *__restrict__ xyz,
-                                                    const double4 *__restrict__ q,
-                                                    const double4 *__restrict__ gx,
-                                                    const double4 *__restrict__ gy,
-                                                    const double4 *__restrict__ gz, double4 *__restrict__ res,
-                                                    uint32_t nfb, uint32_t Nf, const uint32_t *__restrict__ f_node,
-                                                    const double *__restrict__ f_n, const double4 *__restrict__ fq,
-                                                    double U, double V, double4 *__restrict__ fres)
+                                                       const uint32_t *__restrict__ n1,
+                                                       const double4 *__restrict__ egeo,
+                                                       const double4 *__restrict__ xyz,
+                                                       const double4 *__restrict__ q,
+                                                       const double4 *__restrict__ rec, double4 *__restrict__ res,
+                                                       uint32_t nfb, uint32_t Nf, const uint32_t *__restrict__ f_node,
+                                                       const double *__restrict__ f_n, const double4 *__restrict__ fq,
+                                                       double U, double V, double4 *__restrict__ fres)
 {
   if (blockIdx.x < nfb) {
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f < Nf) fres[f] = farfield_flux(U, V, f_n[3 * f], f_n[3 * f + 1], f_n[3 * f + 2], fq[f_node[f]]);
+    if (f < Nf) farfield_store(U, V, f_n + 3 * (size_t)f, fq + f_node[f], fres + f);
     return;
   }
-  const uint32_t e = (blockIdx.x - nfb) * blockDim.x + threadIdx.x;
-  if (e >= E) return;
+  const uint32_t ei = (blockIdx.x - nfb) * blockDim.x + threadIdx.x;
+  const uint32_t e = min(ei, E - 1);   // every lane of a quad takes part
   const uint32_t a = n0[e], o = n1[e];
-  const double4 geo = ldg4(egeo + e);
-  const double4 qa = ldg4(q + a), xa = ldg4(xyz + a), qb = ldg4(q + o), xb = ldg4(xyz + o);
-  const double xm = 0.5 * (xa.x + xb.x), ym = 0.5 * (xa.y + xb.y), zm = 0.5 * (xa.z + xb.z);
+  const double4 geo = ldg4(egeo + e), xa = ldg4(xyz + a), xb = ldg4(xyz + o);
   double4 sL, sR;
   if (FIRST_ORDER) {
+    sL = ldg4(q + a);
+    sR = ldg4(q + o);
+    const double xm = 0.5 * (xa.x + xb.x), ym = 0.5 * (xa.y + xb.y), zm = 0.5 * (xa.z + xb.z);
     const double4 z = make_double4(0, 0, 0, 0);
-    sL = recon(qa, z, z, z, xm - xa.x, ym - xa.y, zm - xa.z);
-    sR = recon(qb, z, z, z, xm - xb.x, ym - xb.y, zm - xb.z);
+    sL = recon(sL, z, z, z, xm - xa.x, ym - xa.y, zm - xa.z);
+    sR = recon(sR, z, z, z, xm - xb.x, ym - xb.y, zm - xb.z);
   } else {
-    const double4 gxa = ldg4(gx + a), gya = ldg4(gy + a), gza = ldg4(gz + a);
-    const double4 gxb = ldg4(gx + o), gyb = ldg4(gy + o), gzb = ldg4(gz + o);
-    sL = recon(qa, gxa, gya, gza, xm - xa.x, ym - xa.y, zm - xa.z);
-    sR = recon(qb, gxb, gyb, gzb, xm - xb.x, ym - xb.y, zm - xb.z);
+    const int lane = threadIdx.x & 31, c = lane & 3, qb = lane & ~3;
+#if KF_FAST
+    const double hx = 0.5 * (xb.x - xa.x), hy = 0.5 * (xb.y - xa.y), hz = 0.5 * (xb.z - xa.z);   // to the midpoint
+#else
+    const double xm = 0.5 * (xa.x + xb.x), ym = 0.5 * (xa.y + xb.y), zm = 0.5 * (xa.z + xb.z);
+    const double hx = xm - xa.x, hy = ym - xa.y, hz = zm - xa.z, kx = xm - xb.x, ky = ym - xb.y, kz = zm - xb.z;
+#endif
+    double4 vL[4], vR[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      vL[i] = ldg4(rec + 4 * (size_t)__shfl_sync(0xffffffffu, a, qb + i) + c);
+      vR[i] = ldg4(rec + 4 * (size_t)__shfl_sync(0xffffffffu, o, qb + i) + c);
+    }
+    double L[4], R[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const double rx = __shfl_sync(0xffffffffu, hx, qb + i), ry = __shfl_sync(0xffffffffu, hy, qb + i),
+                   rz = __shfl_sync(0xffffffffu, hz, qb + i);
+      L[i] = vL[i].x + vL[i].y * rx; L[i] += vL[i].z * ry; L[i] += vL[i].w * rz;
+#if KF_FAST
+      R[i] = vR[i].x - vR[i].y * rx; R[i] -= vR[i].z * ry; R[i] -= vR[i].w * rz;
+#else
+      const double tx = __shfl_sync(0xffffffffu, kx, qb + i), ty = __shfl_sync(0xffffffffu, ky, qb + i),
+                   tz = __shfl_sync(0xffffffffu, kz, qb + i);
+      R[i] = vR[i].x + vR[i].y * tx; R[i] += vR[i].z * ty; R[i] += vR[i].w * tz;
+#endif
+    }
+    quad_transpose(L, c);
+    quad_transpose(R, c);
+    sL = make_double4(L[0], L[1], L[2], L[3]);
+    sR = make_double4(R[0], R[1], R[2], R[3]);
   }
-  res[e] = edge_flux(geo, sL, sR);
+  const double4 f = edge_flux(geo, sL, sR);
+  if (ei < E) stg4(res + ei, f);
 }
 
 // The node pass, four lanes per node, lane c summing flux component c in the
@@ -726,6 +831,9 @@ __global__ void __launch_bounds__(256, 6) k_flux_nodes4(uint32_t N, NodePass a, 
   if (p >= N) return;
   const uint32_t n = a.ord[p];
   const size_t own = 4 * (size_t)n + c;
+  const uint32_t bo = a.bndp[p];
+  uint32_t k = a.in1_ptr[p], e = a.eoff[p];
+  const uint32_t k1 = a.in1_ptr[p + 1], e1 = a.eoff[p + 1];
   double acc = 0.0, jr = 0.0, jw = 0.0, jq = 0.0, jc = 0.0;
   if (JV) {
     jr = a.jr[own];
@@ -733,9 +841,6 @@ __global__ void __launch_bounds__(256, 6) k_flux_nodes4(uint32_t N, NodePass a, 
     jw = a.jwv ? a.jwv[4 * (size_t)p + c] : a.jw[own];
     jc = a.jcdt[n];
   }
-  const uint32_t bo = a.bndp[p];
-  uint32_t k = a.in1_ptr[p];
-  const uint32_t k1 = a.in1_ptr[p + 1], e1 = a.eoff[p + 1];
   for (; k + 4 <= k1; k += 4) {
     double v[4];
 #pragma unroll
@@ -744,7 +849,6 @@ __global__ void __launch_bounds__(256, 6) k_flux_nodes4(uint32_t N, NodePass a, 
     for (int u = 0; u < 4; u++) acc = acc - v[u];
   }
   for (; k < k1; k++) acc = acc - res[4 * (size_t)a.in1_edge[k] + c];
-  uint32_t e = a.eoff[p];
   for (; e + 4 <= e1; e += 4) {
     double v[4];
 #pragma unroll
@@ -2650,25 +2754,19 @@ static void visit_state(DevMesh &m, const double *q)
   kf_count_launch();
 }
 
-// Gradients of q (src/flux.c:60-145) into gx/gy/gz, or into their visit-order
-// copies (m.visit; the residual reads those).  Kernel (KFUN3D_GRADIENT):
-// four lanes per node (default on large meshes), one thread per node with
-// the incidence staged into shared memory by bulk copies (default in the
-// mesh's own order), "plain" one thread per node.
+// Gradients of q (src/flux.c:60-145): for the two-pass residual as the nodes'
+// records (in visit order with m.visit; k_gradient_rec), else into gx/gy/gz,
+// one thread per node, with the incidence staged into shared memory by bulk
+// copies where it fits.  KFUN3D_GRADIENT=plain: not staged.
 void gradient(DevMesh &m, const double *q)
 {
-  if (m.visit) {
-    visit_state(m, q);
-    k_gradient4<<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, nullptr, m.inc_ptr, m.inc_othv, m.inc_w,
-                                                                     m.wstride, (const double *)m.qv,
-                                                                     (double *)m.gxv, (double *)m.gyv,
-                                                                     (double *)m.gzv);
-    kf_count_launch();
-    return;
-  }
-  if (m.grad_lanes == 4) {
-    k_gradient4<<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w,
-                                                                     m.wstride, q, m.gx, m.gy, m.gz);
+  if (m.two_pass) {
+    if (m.visit) visit_state(m, q);
+    const double *Q = m.visit ? (const double *)m.qv : q;
+    const uint32_t *ord = m.visit ? nullptr : m.ord, *oth = m.visit ? m.inc_othv : m.inc_oth;
+    auto kern = m.rec_smem ? k_gradient_rec<true> : k_gradient_rec<false>;
+    if (m.rec_smem) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.rec_smem);
+    kern<<<blocks(m.N, KF_GRAD_NODES), 4 * KF_GRAD_NODES, m.rec_smem, m.stream>>>(m.N, ord, m.inc_ptr, oth, m.inc_w, m.wstride, Q, m.rec, m.status + 1);
     kf_count_launch();
     return;
   }
@@ -2678,27 +2776,21 @@ void gradient(DevMesh &m, const double *q)
       cudaFuncSetAttribute(k_gradient_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       attr_set = true;
     }
-    k_gradient_tma<<<blocks(m.N, 128), 128, m.grad_smem, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride,
-                                                                    (const double4 *)q, (double4 *)m.gx,
-                                                                    (double4 *)m.gy, (double4 *)m.gz, m.status + 1);
+    k_gradient_tma<<<blocks(m.N, 128), 128, m.grad_smem, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride, (const double4 *)q, (double4 *)m.gx, (double4 *)m.gy, (double4 *)m.gz, m.status + 1);
   } else {
-    k_gradient<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride,
-                                                        (const double4 *)q, (double4 *)m.gx,
-                                                        (double4 *)m.gy, (double4 *)m.gz);
+    k_gradient<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride, (const double4 *)q, (double4 *)m.gx, (double4 *)m.gy, (double4 *)m.gz);
   }
   kf_count_launch();
 }
 
-// The gradients in the mesh's numbering (after gradient() wrote visit-order
-// copies), for callers that read them back.
+// The gradients in the mesh's numbering (after gradient() wrote records), for
+// callers that read them back.
 void gradient_to_mesh_order(DevMesh &m)
 {
-  if (!m.visit) return;
-  const unsigned nb = blocks(m.N, 256);
-  k_visit_scatter<<<nb, 256, 0, m.stream>>>(m.N, m.ord, m.gxv, (double4 *)m.gx);
-  k_visit_scatter<<<nb, 256, 0, m.stream>>>(m.N, m.ord, m.gyv, (double4 *)m.gy);
-  k_visit_scatter<<<nb, 256, 0, m.stream>>>(m.N, m.ord, m.gzv, (double4 *)m.gz);
-  kf_count_launch(3);
+  if (!m.two_pass) return;
+  k_unpack_gradient<<<blocks(4 * (size_t)m.N, 256), 256, 0, m.stream>>>(m.N, m.visit ? m.ord : nullptr, m.rec, m.gx,
+                                                                       m.gy, m.gz);
+  kf_count_launch();
 }
 
 // Residual of q into r.  With visit-order copies (m.visit) the edge pass
@@ -2709,21 +2801,13 @@ static void residual_or_jv(DevMesh &m, const double *q, double *r, int first_ord
 {
   if (m.two_pass) {
     if (first_order) visit_state(m, q);
-    const double4 *G[3] = {m.visit ? m.gxv : (const double4 *)m.gx, m.visit ? m.gyv : (const double4 *)m.gy,
-                           m.visit ? m.gzv : (const double4 *)m.gz};
     const double4 *Q = m.visit ? m.qv : (const double4 *)q;
     const double4 *X = m.visit ? m.xyzv : m.xyz;
     const uint32_t *E0 = m.visit ? m.n0v : m.n0s, *E1 = m.visit ? m.n1v : m.n1;
     const uint32_t nfb = blocks(m.Nf, 128);
-    if (nfb + blocks(m.E, 128)) {
-      if (first_order)
-        k_flux_edges<true><<<nfb + blocks(m.E, 128), 128, 0, m.stream>>>(
-            m.E, E0, E1, m.egeo_s, X, Q, nullptr, nullptr, nullptr, m.eres, nfb, m.Nf, m.f_node, m.f_n,
-            (const double4 *)q, u, v, m.fres);
-      else
-        k_flux_edges<false><<<nfb + blocks(m.E, 128), 128, 0, m.stream>>>(
-            m.E, E0, E1, m.egeo_s, X, Q, G[0], G[1], G[2], m.eres, nfb, m.Nf, m.f_node, m.f_n, (const double4 *)q, u, v,
-            m.fres);
+    const unsigned grid = m.E ? nfb + blocks(m.E, 128) : nfb;
+    if (grid) {
+      (first_order ? k_flux_edges<true> : k_flux_edges<false>)<<<grid, 128, 0, m.stream>>>(m.E, E0, E1, m.egeo_s, X, Q, m.rec, m.eres, nfb, m.Nf, m.f_node, m.f_n, (const double4 *)q, u, v, m.fres);
       kf_count_launch();
     }
     NodePass a{m.ord, m.in1_ptr, m.in1_edge, m.eoff, m.bndp, m.bnd_ptr, m.bnd_ent, m.wf_nodes, m.wf_n,

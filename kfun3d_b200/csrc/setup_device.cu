@@ -788,12 +788,13 @@ int kf_build_mesh_lists_device(DevMesh &m, const GEOMETRY *g)
     // its edge geometry, the edges' end points as visit positions, the
     // coordinates in visit order, room for the state and the gradients
     if (ok && m.visit) {
-      ck(cudaMalloc(&m.inc_othv, (ninc + 1) * sizeof(uint32_t)));
+      ck(cudaMalloc(&m.inc_othv, (wst + 4) * sizeof(uint32_t)));   // padded, as inc_oth
+      ck(cudaMemsetAsync(m.inc_othv, 0, (wst + 4) * sizeof(uint32_t), st));
       ck(cudaMalloc(&m.inc_geo, (ninc + 1) * sizeof(double4)));
       ck(cudaMalloc(&m.n0v, E1 * sizeof(uint32_t)));
       ck(cudaMalloc(&m.n1v, E1 * sizeof(uint32_t)));
       ck(cudaMalloc(&m.xyzv, N1 * sizeof(double4)));
-      double4 **vv[] = {&m.qv, &m.gxv, &m.gyv, &m.gzv};
+      double4 **vv[] = {&m.qv};
       for (double4 **v : vv) ck(cudaMalloc(v, N1 * sizeof(double4)));
       if (ok) {
         if (E) {
