@@ -445,6 +445,12 @@ static void release_device(MatrixHandle *h)
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (m->h_scal) cudaFreeHost(m->h_scal);
+  if (m->stage_buf) {
+    if (m->stream) cudaStreamSynchronize(m->stream);   // copies from the buffers may still be queued
+    cudaFreeHost(m->stage_buf);
+  }
+  for (cudaEvent_t e : m->stage_ev)
+    if (e) cudaEventDestroy(e);
   if (m->mgraph) kfun3d_mpnn_graph_free(m->mgraph);
   for (auto &a : m->arnoldi)
     for (auto &b : a)

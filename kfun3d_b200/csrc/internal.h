@@ -134,6 +134,7 @@ const HostPattern &kf_host_pattern(MatrixHandle *h);
 #ifdef __CUDACC__
 
 constexpr int KF_NBASIS = 31;
+constexpr int KF_STAGE_SLOTS = 16;   // pinned buffers of the host copies, two a thread
 
 // Grid-wide barrier for cooperative launches, with a bounded wait.  bar[0]
 // counts arrivals, bar[1] is the generation; both start at zero.  Returns
@@ -361,7 +362,8 @@ struct DevMesh {
                                    // grid barrier between levels, 4 levels with programmatic
                                    // dependent launch (16 lanes/row), 5 one persistent launch,
                                    // 1-3 CTAs per SM, counter barrier, 7 the same with 4 lanes/row,
-                                   // 8 packed level launches (default)
+                                   // 8 the packed factor (default): data-flow sweeps where they
+                                   // fit, else packed level launches
   unsigned trsv_grid = 0;          // persistent grid (whole blocks resident on every SM)
   uint32_t *flags = nullptr;       // [N] per-row completion epoch
   unsigned long long *ticket = nullptr;   // unused (kept zero)
@@ -373,6 +375,11 @@ struct DevMesh {
   double graph_aoa = 0.0;
   bool use_graphs = true;
   double *gs_part = nullptr;      // [64][296] block partial sums, [32][32] lower triangle of the basis' Gram matrix
+  // pinned buffers of large copies from and to the host's arrays (made on
+  // first use), and the event of each one's last copy
+  void *stage_buf = nullptr;
+  cudaEvent_t stage_ev[KF_STAGE_SLOTS] = {};
+  bool stage_used[KF_STAGE_SLOTS] = {}, stage_failed = false;
   // the count of Gram-Schmidt columns written to the host: on the device, in
   // the host's pinned memory (beside h_scal), and as the host expects it
   unsigned *gs_seq_d = nullptr, *h_seq = nullptr, gs_seq = 0;
