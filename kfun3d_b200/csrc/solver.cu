@@ -23,7 +23,7 @@ namespace {
 
 constexpr double JV_EPS = 1.490116119384766e-08;   // src/kernel.c:12
 constexpr int RED_BLOCKS = 296;                    // 2 x 148 SMs
-constexpr int S_XN = 40, S_QN = 42, S_FN = 43, S_T0 = 44, S_CMP = 52;
+constexpr int S_XN = 40, S_QN = 42, S_FN = 43, S_T0 = 44, S_VN = 48, S_CMP = 52;
 
 inline unsigned nblk(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
@@ -332,16 +332,32 @@ __global__ void __launch_bounds__(256, 3) k_gs_update(size_t n, double *__restri
   }
 }
 
-// w /= |w|
-__global__ void __launch_bounds__(256) k_gs_scale(size_t n, double *__restrict__ V, int k, const double *__restrict__ h)
+// w /= |w|, and *xn = |w| of the result: what the next step's difference
+// quotient divides by, without a launch and a pass of its own over the vector
+// (an Arnoldi step at 25^3 130 -> 125 us, 120^3 FP32 1810 -> 1790).  At most
+// eight CTAs an SM, so that few sums are left for the last one.
+__global__ void __launch_bounds__(256) k_gs_scale(size_t n, double *__restrict__ V, int k, const double *__restrict__ h,
+                                                  double *__restrict__ part, unsigned *cnt, double *__restrict__ xn)
 {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n / 2) return;
+  __shared__ double sm[40];
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
   double2 *w = reinterpret_cast<double2 *>(V + (size_t)(k + 1) * n);
   const double sc = 1.0 / h[k + 1];
-  const double2 a = w[i];
-  w[i] = make_double2(a.x * sc, a.y * sc);
+  double s = 0.0;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n / 2; i += stride) {
+    double2 a = w[i];
+    a.x *= sc;
+    a.y *= sc;
+    w[i] = a;
+    s = fma(a.x, a.x, s);
+    s = fma(a.y, a.y, s);
+  }
+  const double bs = block_sum(s, sm);
+  if (threadIdx.x == 0) part[blockIdx.x] = bs;
+  if (!last_cta(cnt)) return;
+  const double t = grid_total(part, gridDim.x, sm);
+  if (threadIdx.x == 0) *xn = sqrt(t);
 }
 
 // Exact-mode modified Gram-Schmidt of V[k+1] against V[0..k] and its
@@ -439,27 +455,28 @@ __global__ void k_scale_inv(size_t n, const double *__restrict__ nrm, double *__
 }
 
 // J.v set-up, src/kernel.c:27-30: h = eps * qnorm; w = (h/|x|) x + q
-__global__ void k_jv_shift(size_t n, const double *__restrict__ scal, const double *__restrict__ x,
-                           const double *__restrict__ q, double *__restrict__ w, int fast)
+__global__ void k_jv_shift(size_t n, const double *__restrict__ xn, const double *__restrict__ qn,
+                           const double *__restrict__ x, const double *__restrict__ q, double *__restrict__ w, int fast)
 {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double h = JV_EPS * scal[S_QN];
-  const double a = h / scal[S_XN];
+  const double h = JV_EPS * qn[0];
+  const double a = h / xn[0];
   w[i] = fast ? fma(a, x[i], q[i]) : a * x[i] + q[i];
 }
 
 // k_jv_shift with the visit-order copy of w written alongside: node i's w in
 // the mesh's order (coalesced, like x and q) and at its visit position
 // rowof[i] in qv (the same arithmetic)
-__global__ void k_jv_shift_visit(uint32_t N, const uint32_t *__restrict__ rowof, const double *__restrict__ scal,
+__global__ void k_jv_shift_visit(uint32_t N, const uint32_t *__restrict__ rowof, const double *__restrict__ xn,
+                                 const double *__restrict__ qn,
                                  const double *__restrict__ x, const double *__restrict__ q, double *__restrict__ w,
                                  double4 *__restrict__ qv, int fast)
 {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double h = JV_EPS * scal[S_QN];
-  const double a = h / scal[S_XN];
+  const double h = JV_EPS * qn[0];
+  const double a = h / xn[0];
   const double4 xx = reinterpret_cast<const double4 *>(x)[i], qq = reinterpret_cast<const double4 *>(q)[i];
   double4 o;
   o.x = fast ? fma(a, xx.x, qq.x) : a * xx.x + qq.x;
@@ -640,24 +657,27 @@ void dev_residual(DevMesh &m, const Ops &o, const double *q, double *r)
   o.residual(m, q, r, fo, u, v);
 }
 
-// iJacVec, src/kernel.c:24-45: y = (F(q + h x/|x|) - r + cdt (w - q)) |x| / h
-void dev_jacvec(DevMesh &m, const Ops &o, const double *x, double *y)
+// iJacVec, src/kernel.c:24-45: y = (F(q + h x/|x|) - r + cdt (w - q)) |x| / h;
+// vnorm: x is the basis vector that the last gram_schmidt normalised, its norm
+// is in S_VN.
+void dev_jacvec(DevMesh &m, const Ops &o, const double *x, double *y, bool vnorm = false)
 {
   const size_t n = 4 * (size_t)m.N;
-  dev_reduce(m, x, x, m.scal + S_XN, 1, o.fast);
+  const double *xn = m.scal + (vnorm ? S_VN : S_XN), *qn = m.scal + S_QN;
+  if (!vnorm) dev_reduce(m, x, x, m.scal + S_XN, 1, o.fast);
   if (m.visit) {
     // the shifted state and its visit-order copy in one pass
-    k_jv_shift_visit<<<nblk(m.N, 256), 256, 0, m.stream>>>(m.N, m.rowof, m.scal, x, m.q, m.w, m.qv, o.fast);
+    k_jv_shift_visit<<<nblk(m.N, 256), 256, 0, m.stream>>>(m.N, m.rowof, xn, qn, x, m.q, m.w, m.qv, o.fast);
     m.qv_of = m.w;
   } else {
-    k_jv_shift<<<nblk(n, 256), 256, 0, m.stream>>>(n, m.scal, x, m.q, m.w, o.fast);
+    k_jv_shift<<<nblk(n, 256), 256, 0, m.stream>>>(n, xn, qn, x, m.q, m.w, o.fast);
   }
   kf_count_launch();
   double u, v;
   kfun3d_get_freestream(&u, &v);
   const int fo = kf_first_order();
   if (!fo) o.gradient(m, m.w);
-  o.residual_jv(m, m.w, y, fo, u, v, JvArgs{m.r, m.q, m.scal + S_XN, m.scal + S_QN, JV_EPS});
+  o.residual_jv(m, m.w, y, fo, u, v, JvArgs{m.r, m.q, xn, qn, JV_EPS});
 }
 
 void dev_axpy(DevMesh &m, double a, const double *x, double *y, bool fast)
@@ -713,7 +733,8 @@ void gram_schmidt(DevMesh &m, int k)
   launch_dependent(k_gs_update, grid, m.stream, n, m.V, k, m.scal, m.gs_part, m.bar + 3, m.h_scal, m.gs_seq_d,
                    (volatile unsigned *)m.h_seq);
   m.gs_seq++;
-  launch_dependent(k_gs_scale, std::max(1u, nblk(n / 2, 256)), m.stream, n, m.V, k, (const double *)m.scal);
+  launch_dependent(k_gs_scale, std::min(1184u, std::max(1u, nblk(n / 2, 256))), m.stream, n, m.V, k,
+                   (const double *)m.scal, m.gs_part, m.bar + 6, m.scal + S_VN);
   kf_count_launch(3);
 }
 
@@ -732,7 +753,7 @@ void orthogonalize(DevMesh &m, const Ops &o, int k)
 // orthogonalised and normalised; h in scal[0..k+1].
 void arnoldi_step(DevMesh &m, const Ops &o, int k, int prec)
 {
-  dev_jacvec(m, o, Vb(m, k), m.t);
+  dev_jacvec(m, o, Vb(m, k), m.t, o.fast && k > 0);   // (V[0]: normalised by dev_normalize)
   o.sptrsv(m, m.t, Vb(m, k + 1), prec);
   orthogonalize(m, o, k);
 }
@@ -1725,6 +1746,7 @@ extern "C" double kfun3d_time_kernel(GEOMETRY *g, int which, int reps)
     CK(cudaMemcpyAsync(Vb(*m, k), m->r, n * sizeof(double), cudaMemcpyDeviceToDevice, m->stream));
     dev_normalize(*m, Vb(*m, k), m->scal + S_T0, o.fast);
   }
+  dev_reduce(*m, Vb(*m, 15), Vb(*m, 15), m->scal + S_VN, 1, o.fast);   // for arnoldi_step
   auto run = [&]() {
     switch (which) {
       case 0: dev_residual(*m, o, m->q, m->r); break;
