@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(128) k_residual(uint32_t N, const uint32_t *__
 // edge's state.  With a lane reading the state and the gradients of its own
 // edge's ends, each in a request of its own, the L1 data path was 75 % busy and
 // bounded the kernel.  Edges and nodes at 70^3 142 -> 123 us, at 120^3 522 -> 515
-// (there the 384 MB of edge fluxes, written once and read twice, take 173 us at
+// (with the node pass of that time; there the 384 MB of edge fluxes, written once and read twice, take 173 us at
 // a copy's rate); seven CTAs an SM (at 120^3 six take 550 us, five 581, eight 524
 // with the records loaded in two halves).
 // (not inlined: its registers are not the edges')
@@ -814,6 +814,12 @@ __global__ void __launch_bounds__(128, 7) k_flux_edges(uint32_t E, const uint32_
 // fluxes (src/flux.c:541-779) in list order.  JV: the sum y is not stored but
 // (y - r + cdt (w - q)) |x| / h, the Jacobian-vector product of
 // src/kernel.c:35-44 (w in visit order when wv is given).
+// Bound by the latency of the fluxes' gathers (DRAM a quarter busy): up to eight
+// of each side are asked for before the first is used; a node has about seven a
+// side, the rest follow one by one.  Edges and nodes with four of one side at a
+// time / so: 70^3 123 / 115 us, 120^3 515 / 485; the Arnoldi step at 120^3 1790 /
+// 1766 (JV: its own loads only once half of the batch is summed, so that six CTAs
+// an SM fit; loaded first, with five: 1776).
 struct NodePass {
   const uint32_t *ord, *in1_ptr, *in1_edge, *eoff;
   const uint32_t *bndp, *bnd_ptr, *bnd_ent, *wf_nodes;
@@ -835,28 +841,25 @@ __global__ void __launch_bounds__(256, 6) k_flux_nodes4(uint32_t N, NodePass a, 
   uint32_t k = a.in1_ptr[p], e = a.eoff[p];
   const uint32_t k1 = a.in1_ptr[p + 1], e1 = a.eoff[p + 1];
   double acc = 0.0, jr = 0.0, jw = 0.0, jq = 0.0, jc = 0.0;
+  double v[8], w[8];
+#pragma unroll
+  for (int u = 0; u < 8; u++) v[u] = k + u < k1 ? res[4 * (size_t)a.in1_edge[k + u] + c] : 0.0;
+#pragma unroll
+  for (int u = 0; u < 8; u++) w[u] = e + u < e1 ? res[4 * (size_t)(e + u) + c] : 0.0;
+#pragma unroll
+  for (int u = 0; u < 8; u++)
+    if (k + u < k1) acc = acc - v[u];
+  for (k += 8; k < k1; k++) acc = acc - res[4 * (size_t)a.in1_edge[k] + c];
   if (JV) {
     jr = a.jr[own];
     jq = a.jq[own];
     jw = a.jwv ? a.jwv[4 * (size_t)p + c] : a.jw[own];
     jc = a.jcdt[n];
   }
-  for (; k + 4 <= k1; k += 4) {
-    double v[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) v[u] = res[4 * (size_t)a.in1_edge[k + u] + c];
-#pragma unroll
-    for (int u = 0; u < 4; u++) acc = acc - v[u];
-  }
-  for (; k < k1; k++) acc = acc - res[4 * (size_t)a.in1_edge[k] + c];
-  for (; e + 4 <= e1; e += 4) {
-    double v[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) v[u] = res[4 * (size_t)(e + u) + c];
-#pragma unroll
-    for (int u = 0; u < 4; u++) acc = acc + v[u];
-  }
-  for (; e < e1; e++) acc = acc + res[4 * (size_t)e + c];
+  for (int u = 0; u < 8; u++)
+    if (e + u < e1) acc = acc + w[u];
+  for (e += 8; e < e1; e++) acc = acc + res[4 * (size_t)e + c];
   if (bo != 0xffffffffu)
     for (uint32_t b = a.bnd_ptr[bo]; b < a.bnd_ptr[bo + 1]; b++) {
       const uint32_t ent = a.bnd_ent[b], kind = ent >> 29, idx = ent & 0x1fffffffu;
