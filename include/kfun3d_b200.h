@@ -270,16 +270,18 @@ long kfun3d_matrix_read(const GEOMETRY *g, unsigned int *ia, unsigned int *ja, d
    GEOMETRY, in the mesh's ILU(0) order and in the precision that is still
    set (a changed kfun3d_set_precision or the spatial order is refused with
    KFUN3D_ERR_ARG); d_b and d_x are the caller's device arrays of 4*nnodes
-   doubles (16-byte aligned, distinct).  Runs the sync-free sweep, whose
-   per-row completion flags live in a fixed device array of the library
-   (8 MiB, held by every GPU that loads the library until exit, cleared by
-   each call), so the call allocates nothing; at most 2,097,152 rows, larger
-   matrices are rejected (KFUN3D_ERR_ARG).  The first call on a device looks
-   up that array's device address (cudaGetSymbolAddress).  The call waits for
+   doubles (16-byte aligned, distinct).  Runs the data-flow sweeps on
+   buffers the device mirror already holds, or, for a matrix they do not take
+   (rows of more than 96 blocks), the sync-free sweep, whose per-row completion
+   flags live in a fixed device array of the library (8 MiB, held by every GPU
+   that loads the library until exit, cleared by each call), so the call
+   allocates nothing; at most 2,097,152 rows, larger matrices are rejected
+   (KFUN3D_ERR_ARG).  The first call on a device looks up that array's device
+   address (cudaGetSymbolAddress).  The call waits for
    all work already queued on the device (so b may be written on any stream
    just before), runs on the library's stream and returns once x is written.
-   Calls share the array: calls that overlap on the GPU (from several host
-   threads) race.  Returns KFUN3D_OK or an error code (also recorded). */
+   Calls share the array and the mirror's buffers: calls that overlap on the
+   GPU (from several host threads) race.  Returns KFUN3D_OK or an error code (also recorded). */
 int kfun3d_sptrsv_device_noalloc(const GEOMETRY *g, const double *d_b, double *d_x);
 
 /* Release the device mirror of g (also done by CXX_Matrix_Delete). */
@@ -297,12 +299,13 @@ int kfun3d_check_bounded_wait(void);
 
 /* Which device paths g's mirror uses (for tests and reports; builds the
    mirror on first use): key "sptrsv_schedule" -> the triangular-solve
-   schedule of the active ILU(0) order (8 packed level launches, 7 four-lane
-   level launches, ...), "lsq_terms_match" -> 1 when the least-squares
+   schedule of the active ILU(0) order (8 the packed factor: both sweeps in one
+   data-flow launch, or level launches where a row is too long for it or
+   KFUN3D_SPTRSV=packed asks for them; 7 four-lane level launches, ...), "lsq_terms_match" -> 1 when the least-squares
    terms recomputed on the device from per-node coefficients made there equal
    the GEOMETRY's stored terms bit for bit, "visit_order_copies" -> 1 when
    the residual passes work on copies of the node data in their spatial visit
-   order, "mgs_resident" -> 1 when Gram-Schmidt keeps the vector on chip,
+   order, "mgs_resident" -> 0 (no kernel keeps the vector on chip any more),
    "pattern_matches_host" / "spatial_pattern_matches_host" -> 1 when the
    block pattern, level lists and ILU(0) product lists built on the device
    (mesh numbering / spatial renumbering; -1 while the latter is not built)

@@ -365,7 +365,7 @@ class Mesh:
 
     def query(self, key):
         """Device path in use (kfun3d_device_query): "sptrsv_schedule", "lsq_terms_match",
-        "visit_order_copies", "mgs_resident"."""
+        "visit_order_copies"."""
         v = lib().kfun3d_device_query(self.g, key.encode())
         if v < 0:
             raise RuntimeError(f"kfun3d_device_query({key}) failed: {last_error()}")

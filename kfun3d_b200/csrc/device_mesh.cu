@@ -440,7 +440,7 @@ static void release_device(MatrixHandle *h)
                   m->wf_n, m->s_n, m->f_n, m->bnd_of, m->bndp, m->f_node, m->fres, m->bnd_node, m->bnd_ptr, m->bnd_ent, m->ia, m->ja,
                   m->diag, m->tblk, m->lpos, m->last_lower, m->lev_l, m->lev_u, m->A, m->lslot, m->dinv,
                   m->Af, m->dinvf, m->q, m->r, m->gx, m->gy, m->gz, m->cdt, m->w, m->t, m->x, m->rhs, m->V,
-                  m->red, m->scal, m->forces, m->dscr, m->status, m->flags, m->ticket, m->gs_part, m->gs_seq_d, m->lsq_coef,
+                  m->red, m->scal, m->forces, m->dscr, m->status, m->flags, m->gs_part, m->gs_seq_d, m->lsq_coef,
                   m->qv, m->xyzv, m->rec, m->inc_othv, m->n0v, m->n1v, m->inc_geo, m->desc_l, m->desc_u, m->eoff, m->n1, m->in1_ptr, m->in1_edge, m->eres, m->n0s, m->pair_ptr, m->pairs, m->lev_ptr_d, m->bar, m->Z, m->qold, m->fy, m->fx, m->pscr, m->ord, m->rowof, m->egeo_s, m->sub_part};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -899,8 +899,6 @@ DevMesh *kf_device(const GEOMETRY *g)
   KF_CUDA(cudaMemset(m->status, 0, 4 * sizeof(int)));
   KF_CUDA(cudaMalloc(&m->flags, (size_t)N * sizeof(uint32_t)));
   KF_CUDA(cudaMemset(m->flags, 0, (size_t)N * sizeof(uint32_t)));
-  KF_CUDA(cudaMalloc(&m->ticket, sizeof(unsigned long long)));
-  KF_CUDA(cudaMemset(m->ticket, 0, sizeof(unsigned long long)));
   {
     int nsm = 0;
     KF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device));

@@ -366,7 +366,6 @@ struct DevMesh {
                                    // fit, else packed level launches
   unsigned trsv_grid = 0;          // persistent grid (whole blocks resident on every SM)
   uint32_t *flags = nullptr;       // [N] per-row completion epoch
-  unsigned long long *ticket = nullptr;   // unused (kept zero)
   uint4 *desc_l = nullptr, *desc_u = nullptr;   // [N] (row, first block, end block) in level order
   // fast mode: one CUDA graph per Arnoldi index (jacobian-vector product,
   // triangular solves, Gram-Schmidt, read-back of the Hessenberg column)

@@ -7,13 +7,14 @@
 // cudaMalloc afterwards).  ComputeSparseTriangularSolve takes host arrays and
 // stages them through buffers of the GEOMETRY's device mirror;
 // kfun3d_sptrsv_device_noalloc instead takes the caller's device arrays and
-// keeps its only working memory -- the per-row completion flags of the
-// sync-free sweep -- in a fixed, file-scope device array, so the call itself
-// allocates nothing.
+// allocates nothing: the data-flow sweeps work in buffers the mirror already
+// holds, and the sync-free sweep, for matrices with rows too long for those,
+// keeps its only working memory -- the per-row completion flags -- in a fixed,
+// file-scope device array.
 //
 // Ordering: the call first waits for all work already queued on the device
-// (so the caller's writes of b, on any stream, are complete), runs the sweep
-// on the library's stream and waits for it before returning (so x is final
+// (so the caller's writes of b, on any stream, are complete), runs the sweeps
+// on the library's stream and waits for them before returning (so x is final
 // when the call returns).
 #include <cstdio>
 #include <cstring>
