@@ -1387,9 +1387,11 @@ struct HostCopy {
 // (about 5 GB/s into pages not yet touched; one residual of the 70^3 mesh, 11 MB
 // in and 44 MB out: 10.3 -> 5.2 ms).  To the host, the arrays are written when
 // the call returns; to the device, the copies are queued on the mesh's stream.
-// From 4 MB; the buffers (16 MB) are the mesh's and go with it.  A chunk a
+// From 32 MB: shorter copies do not repay the threads' start (four calls that
+// copy 8 MB each way at 63^3: 5.9 ms staged, 5.5 directly).  The buffers (16 MB)
+// are the mesh's and go with it.  A chunk a
 // buffer, two buffers a thread; the threads take chunks in turn.
-constexpr size_t STAGE_MIN = 4u << 20, STAGE_CHUNK = 1u << 20;
+constexpr size_t STAGE_MIN = 32u << 20, STAGE_CHUNK = 1u << 20;
 
 bool stage_ready(DevMesh &m)
 {
