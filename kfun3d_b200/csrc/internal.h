@@ -396,6 +396,8 @@ struct DevMesh {
   int pk_cut[2] = {0, 0};         // chunk cut used with FP64 / FP32 factors (0: 32 rows, 1: 64 rows)
   bool pk_fp64 = false;           // FP64 factors also take the packed schedule (KFUN3D_PK_FP64=1)
   void *pk_buf = nullptr;         // the packed factor: lower stream, then upper stream (FP64 or FP32 blocks)
+  int pk_precision = -1;          // the precision whose blocks it holds (-1: none, or the matrix has changed since)
+  int pk_order = -1;              // and their elimination order (ilu_active)
   // data-flow sweeps over the packed factor (k_trsv_flow): rows wait for the
   // values they read instead of for levels
   bool pk_flow = true;            // used by mode 8 where the rows fit (KFUN3D_SPTRSV=packed: level launches)

@@ -2900,6 +2900,7 @@ void fill(DevMesh &m, const double *q, double u, double v, int precision)
                                                                m.fill_lpos, A, lslot, m.bnd_of, dscr);
   };
   if (precision == 0) {
+    if (m.pk_precision == 0) m.pk_precision = -1;   // an FP64 solve reads the matrix as it now stands
     fill_fn(m.A, m.lslot, nullptr);
     kf_count_launch();
     if (m.nb) {
@@ -2921,6 +2922,33 @@ void fill(DevMesh &m, const double *q, double u, double v, int precision)
 }
 
 static void packed_setup();
+
+// The packed copy (m.pk_buf) of the matrix in the given precision and the
+// active order.  There is one copy, the precision and order it holds beside it.
+static void pack_factor(DevMesh &m, int precision)
+{
+  for (int pass = 0; pass < 2; pass++) {
+    const uint32_t nb = m.pk[pass].nblk, off = pass == 0 ? 0u : m.pk[0].nblk;
+    if (precision == 0)
+      k_trsv_pack<double><<<blocks((size_t)nb * 8, 256), 256, 0, m.stream>>>(
+          nb, m.pk[pass].src, m.A, reinterpret_cast<double *>(m.pk_buf) + 16 * (size_t)off);
+    else
+      k_trsv_pack<float><<<blocks((size_t)nb * 4, 256), 256, 0, m.stream>>>(
+          nb, m.pk[pass].src, m.Af, reinterpret_cast<float *>(m.pk_buf) + 16 * (size_t)off);
+    kf_count_launch();
+  }
+  m.pk_precision = precision;
+  m.pk_order = m.ilu_active;
+}
+
+// Before sweeps over the packed copy: made again when it holds another
+// precision's or order's blocks, or when the matrix was filled after it.  (A
+// solve factors, which packs, before it captures its steps: no captured graph
+// holds these launches.)
+static void packed_current(DevMesh &m, int precision)
+{
+  if (m.pk_precision != precision || m.pk_order != m.ilu_active) pack_factor(m, precision);
+}
 
 // The data-flow sweeps serve the active pattern: mode 8, and no row longer
 // than their shared-memory stage.
@@ -2991,19 +3019,7 @@ void ilu(DevMesh &m, int precision)
   else
     k_ilu_finish_f32<<<blocks((size_t)m.N * 16, 256), 256, 0, m.stream>>>(m.N, m.diag, m.dinvf, m.Af);
   kf_count_launch();
-  if (m.trsv_mode == 8 && m.pk[0].chunk[0] && (precision == 1 || m.pk_fp64 || flow_fits(m))) {
-    packed_setup();
-    for (int pass = 0; pass < 2; pass++) {
-      const uint32_t nb = m.pk[pass].nblk, off = pass == 0 ? 0u : m.pk[0].nblk;
-      if (precision == 0)
-        k_trsv_pack<double><<<blocks((size_t)nb * 8, 256), 256, 0, m.stream>>>(
-            nb, m.pk[pass].src, m.A, reinterpret_cast<double *>(m.pk_buf) + 16 * (size_t)off);
-      else
-        k_trsv_pack<float><<<blocks((size_t)nb * 4, 256), 256, 0, m.stream>>>(
-            nb, m.pk[pass].src, m.Af, reinterpret_cast<float *>(m.pk_buf) + 16 * (size_t)off);
-      kf_count_launch();
-    }
-  }
+  if (m.trsv_mode == 8 && m.pk[0].chunk[0] && (precision == 1 || m.pk_fp64 || flow_fits(m))) pack_factor(m, precision);
 }
 
 // Dynamic shared memory of k_trsv_packed for a chunk of `blocks` blocks.
@@ -3048,6 +3064,7 @@ static void sptrsv_packed(DevMesh &m, const double *b, double *x, const uint32_t
                           double *xout = nullptr)
 {
   packed_setup();
+  packed_current(m, sizeof(T) == 8 ? 0 : 1);
   int *err = m.status + 1;
   const T *base = reinterpret_cast<const T *>(m.pk_buf);
   const int cut = m.pk_cut[sizeof(T) == 8 ? 0 : 1];
@@ -3091,6 +3108,7 @@ static void sptrsv_packed(DevMesh &m, const double *b, double *x, const uint32_t
 // mesh's numbering whatever the pattern's.
 template <typename T> static void sptrsv_flow(DevMesh &m, const double *b, double *x)
 {
+  packed_current(m, sizeof(T) == 8 ? 0 : 1);
   const void *fn = m.flow_lanes == 8 ? (const void *)k_trsv_flow<T, 8, 4, sizeof(T) == 4 ? 5 : 4>
                                        : (const void *)k_trsv_flow<T, 4, 8, sizeof(T) == 4 ? 4 : 3>;
   cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
