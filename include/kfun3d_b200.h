@@ -291,8 +291,9 @@ void kfun3d_device_release(GEOMETRY *g);
    waits, the way the sync-free triangular sweep waits for a row, on a flag
    that nothing sets, and must give up after the library's poll limit (about
    a second at most); a second wait on a flag that is set must return at once,
-   in the same context.  Returns KFUN3D_ERR_TIMEOUT when both behave so,
-   KFUN3D_ERR_ARG when either does not, KFUN3D_ERR_CUDA / _NO_DEVICE on a
+   in the same context; and a wait for copies whose arrival comes only after it
+   has given up must still see the arrival out.  Returns KFUN3D_ERR_TIMEOUT when
+   all behave so, KFUN3D_ERR_ARG when one does not, KFUN3D_ERR_CUDA / _NO_DEVICE on a
    CUDA failure or without a device.  For tests and bring-up; no counterpart
    in the reference. */
 int kfun3d_check_bounded_wait(void);

@@ -299,20 +299,22 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
 constexpr uint32_t KF_MBAR_LIMIT = 1u << 24;
 
 // Bounded wait for phase `phase` of the mbarrier; false (and *err set) if it
-// gave up.
-__device__ __forceinline__ bool mbar_wait(uint64_t *mbar, unsigned phase, int *err)
+// gave up.  It gives up in two steps of `limit` polls: after the first *err is
+// set, in the second the copies may still land, so that a CTA does not return
+// while they are on their way into its shared memory.
+__device__ __forceinline__ bool mbar_wait(uint64_t *mbar, unsigned phase, int *err, uint32_t limit = KF_MBAR_LIMIT)
 {
   const unsigned a = smem_addr(mbar);
-  for (uint32_t spins = 0; spins < KF_MBAR_LIMIT; spins++) {
+  for (uint32_t spins = 0; spins < 2 * limit; spins++) {
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done)
         : "r"(a), "r"(phase)
         : "memory");
-    if (done) return true;
+    if (done) return spins < limit;
+    if (spins == limit - 1) atomicExch(err, 1);
   }
-  atomicExch(err, 1);
   return false;
 }
 
@@ -2507,9 +2509,11 @@ struct FlowSweep {
 // shared-memory stage (mbarrier, bounded wait), its slots into registers.
 //
 // Progress: every CTA is resident (cooperative launch), and a warp waits only
-// for rows of earlier chunks, whose warps work theirs in order.  A wait that
-// gives up sets *err; the warp then runs through its remaining chunks without
-// waiting, so that no copy is left in flight.
+// for rows of earlier chunks, whose warps work theirs in order.  A wait for a
+// value that gives up sets *err; the warp then runs through its remaining
+// chunks without waiting for values.  A wait for a chunk's copies that gives up
+// sets *err too; the warp then stops, once the copies of both its stages have
+// landed (or as long a wait again has passed).
 //
 // Buffers: y and the x of this solve must be KF_FLOW_EMPTY on entry.  The upper
 // sweep's row clears its y once it has every x it reads (the rows that read
@@ -2584,7 +2588,11 @@ __global__ void __launch_bounds__(128, MINB)
     const size_t own = 4 * (size_t)s0.x + r;
     double xi = 0.0;
     if (active && !upper) xi = b[4 * (size_t)s0.w + r];
-    if (!__all_sync(0xffffffffu, mbar_wait(&mbars[warp][st], phase, err))) break;
+    if (!__all_sync(0xffffffffu, mbar_wait(&mbars[warp][st], phase, err))) {
+      // the other stage's copies, issued for the chunk after this one, land first
+      if (c + W < total) mbar_wait(&mbars[warp][st ^ 1], phase ^ (uint32_t)st, err);
+      break;
+    }
     const unsigned char *sg = stage0 + (size_t)st * stage_bytes;
     const T *sa = reinterpret_cast<const T *>(sg) + 4 * r;
     const uint32_t *sc = reinterpret_cast<const uint32_t *>(sg + (size_t)stage_blk * 16 * sizeof(T)) + (d0.z & 3u);
@@ -3055,6 +3063,29 @@ __global__ void k_wait_on_flag(const uint32_t *flag, uint32_t value, int *err)
   }
 }
 
+// mbar_wait on a barrier whose one arrival comes only after the wait has given
+// up (*err set): the wait then has to see it out.  out[0] what the wait
+// returned, out[1] whether the arrival came before it did.
+__global__ void k_late_arrival(int *err, int *out)
+{
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ volatile int landed;
+  if (threadIdx.x == 0) {
+    mbar_init(&mbar, 1);
+    landed = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    out[0] = mbar_wait(&mbar, 0, err, 1024);
+    out[1] = landed;
+  } else if (threadIdx.x == 32) {
+    for (uint32_t spins = 0; spins < KF_SPIN_LIMIT && !*(volatile int *)err; spins++) {}
+    landed = 1;
+    __threadfence_block();
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&mbar)) : "memory");
+  }
+}
+
 // Both sweeps of the packed schedule: one launch per level, chained by
 // programmatic dependent launch (the first level of the lower sweep waits for
 // the right-hand side normally).  The chunk cut (32 or 64 rows a CTA) is the
@@ -3167,23 +3198,25 @@ bool sptrsv_permuted(DevMesh &m, const double *b, double *x, int precision)
 
 // The device-side bounded waits at work without a fault: a wait on a flag
 // that nothing sets must give up (KFUN3D_ERR_TIMEOUT), and the same wait on a
-// set flag must return at once, in the same context.  Anything else is an
-// error code (KFUN3D_ERR_CUDA for a CUDA failure, KFUN3D_ERR_ARG if either
-// wait behaved otherwise).
+// set flag must return at once, in the same context; a wait for an arrival that
+// comes after it has given up must not return before it.  Anything else is an
+// error code (KFUN3D_ERR_CUDA for a CUDA failure, KFUN3D_ERR_ARG if a wait
+// behaved otherwise).
 int bounded_wait_check(cudaStream_t st)
 {
   uint32_t *flag = nullptr;
   int *err = nullptr;
-  int h[2] = {0, 0};
-  bool ok = cudaMalloc(&flag, sizeof(uint32_t)) == cudaSuccess && cudaMalloc(&err, 2 * sizeof(int)) == cudaSuccess;
+  int h[5] = {0, 0, 0, 0, 0};
+  bool ok = cudaMalloc(&flag, sizeof(uint32_t)) == cudaSuccess && cudaMalloc(&err, sizeof(h)) == cudaSuccess;
   ok = ok && cudaMemsetAsync(flag, 0, sizeof(uint32_t), st) == cudaSuccess &&
-       cudaMemsetAsync(err, 0, 2 * sizeof(int), st) == cudaSuccess;
+       cudaMemsetAsync(err, 0, sizeof(h), st) == cudaSuccess;
   if (ok) {
     k_wait_on_flag<<<1, 32, 0, st>>>(flag, 1u, err);       // nothing sets it: gives up
     k_wait_on_flag<<<1, 32, 0, st>>>(flag, 0u, err + 1);   // already set: returns at once
-    kf_count_launch(2);
+    k_late_arrival<<<1, 64, 0, st>>>(err + 2, err + 3);    // gives up, but sees the arrival out
+    kf_count_launch(3);
     ok = cudaGetLastError() == cudaSuccess &&
-         cudaMemcpyAsync(h, err, 2 * sizeof(int), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+         cudaMemcpyAsync(h, err, sizeof(h), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
          cudaStreamSynchronize(st) == cudaSuccess;
   }
   if (flag) cudaFree(flag);
@@ -3192,7 +3225,8 @@ int bounded_wait_check(cudaStream_t st)
     cudaGetLastError();
     return KFUN3D_ERR_CUDA;
   }
-  return (h[0] == 1 && h[1] == 0) ? KFUN3D_ERR_TIMEOUT : KFUN3D_ERR_ARG;
+  const bool late = h[2] == 1 && h[3] == 0 && h[4] == 1;
+  return (h[0] == 1 && h[1] == 0 && late) ? KFUN3D_ERR_TIMEOUT : KFUN3D_ERR_ARG;
 }
 
 void sptrsv(DevMesh &m, const double *b, double *x, int precision)

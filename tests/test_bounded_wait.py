@@ -1,8 +1,10 @@
 """Failure detection without a GPU fault: the device-side waits of the
 library (the sync-free triangular sweep's row flags, the grid barriers of
-the cooperative kernels) are bounded.  A wait on a flag that nothing sets
-gives up after the poll limit and reports it, and the context stays usable:
-the library's kernels run bit-identically afterwards."""
+the cooperative kernels, the barriers of copies into shared memory) are
+bounded.  A wait on a flag that nothing sets gives up after the poll limit and
+reports it, one whose copies land late reports it too but sees them out first,
+and the context stays usable: the library's kernels run bit-identically
+afterwards."""
 import numpy as np
 import pytest
 
