@@ -302,11 +302,12 @@ int kfun3d_check_bounded_wait(void);
    mirror on first use): key "sptrsv_schedule" -> the triangular-solve
    schedule of the active ILU(0) order (8 the packed factor: both sweeps in one
    data-flow launch, or level launches where a row is too long for it or
-   KFUN3D_SPTRSV=packed asks for them; 7 four-lane level launches, ...), "lsq_terms_match" -> 1 when the least-squares
-   terms recomputed on the device from per-node coefficients made there equal
-   the GEOMETRY's stored terms bit for bit, "visit_order_copies" -> 1 when
-   the residual passes work on copies of the node data in their spatial visit
-   order, "mgs_resident" -> 0 (no kernel keeps the vector on chip any more),
+   KFUN3D_SPTRSV=packed asks for them; 7 four-lane level launches, ...),
+   "sptrsv_flow" -> 1 when that is the data-flow launch, "lsq_terms_match" -> 1
+   when the least-squares terms recomputed on the device from per-node
+   coefficients made there equal the GEOMETRY's stored terms bit for bit,
+   "visit_order_copies" -> 1 when the residual passes work on copies of the
+   node data in their spatial visit order, "mgs_resident" -> 0 (no kernel keeps the vector on chip any more),
    "pattern_matches_host" / "spatial_pattern_matches_host" -> 1 when the
    block pattern, level lists and ILU(0) product lists built on the device
    (mesh numbering / spatial renumbering; -1 while the latter is not built)

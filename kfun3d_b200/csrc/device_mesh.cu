@@ -588,6 +588,7 @@ extern "C" long kfun3d_device_query(const GEOMETRY *g, const char *key)
   DevMesh *m = key ? kf_device(g) : nullptr;
   if (!m) return -1;
   if (strcmp(key, "sptrsv_schedule") == 0) return m->trsv_mode;
+  if (strcmp(key, "sptrsv_flow") == 0) return kf_flow_fits(*m) ? 1 : 0;
   if (strcmp(key, "lsq_terms_match") == 0) return m->lsq_match ? 1 : 0;
   if (strcmp(key, "visit_order_copies") == 0) return m->visit ? 1 : 0;
   if (strcmp(key, "mgs_resident") == 0) return 0;   // (no Gram-Schmidt kernel keeps the vector on chip any more)

@@ -445,6 +445,14 @@ std::vector<uint32_t> kf_partition_rcb(const double *X, const double *Y, const d
 void kf_count_launch(unsigned n = 1);
 void kfun3d_reset_launch_count_by(unsigned long long n);   // undo counts taken during graph capture
 
+// The data-flow sweeps serve the active pattern: mode 8, and no row longer
+// than their shared-memory stage.
+inline bool kf_flow_fits(const DevMesh &m)
+{
+  return m.pk_flow && m.trsv_mode == 8 && m.pk[0].chunk[2] && m.pk[1].chunk[2] &&
+         std::max(m.pk[0].maxblk[2], m.pk[1].maxblk[2]) <= KF_FLOW_ROW_MAX;
+}
+
 // Clears the data-flow sweeps' buffers to "not written" (at set-up, and after
 // a wait that gave up).
 cudaError_t kf_flow_reset(DevMesh &m);

@@ -2958,14 +2958,6 @@ static void packed_current(DevMesh &m, int precision)
   if (m.pk_precision != precision || m.pk_order != m.ilu_active) pack_factor(m, precision);
 }
 
-// The data-flow sweeps serve the active pattern: mode 8, and no row longer
-// than their shared-memory stage.
-static bool flow_fits(const DevMesh &m)
-{
-  return m.pk_flow && m.trsv_mode == 8 && m.pk[0].chunk[2] && m.pk[1].chunk[2] &&
-         std::max(m.pk[0].maxblk[2], m.pk[1].maxblk[2]) <= KF_FLOW_ROW_MAX;
-}
-
 void ilu(DevMesh &m, int precision)
 {
   int *status = m.status;
@@ -3027,7 +3019,7 @@ void ilu(DevMesh &m, int precision)
   else
     k_ilu_finish_f32<<<blocks((size_t)m.N * 16, 256), 256, 0, m.stream>>>(m.N, m.diag, m.dinvf, m.Af);
   kf_count_launch();
-  if (m.trsv_mode == 8 && m.pk[0].chunk[0] && (precision == 1 || m.pk_fp64 || flow_fits(m))) pack_factor(m, precision);
+  if (m.trsv_mode == 8 && m.pk[0].chunk[0] && (precision == 1 || m.pk_fp64 || kf_flow_fits(m))) pack_factor(m, precision);
 }
 
 // Dynamic shared memory of k_trsv_packed for a chunk of `blocks` blocks.
@@ -3134,7 +3126,7 @@ static void sptrsv_packed(DevMesh &m, const double *b, double *x, const uint32_t
   }
 }
 
-// Both sweeps through k_trsv_flow (flow_fits): one cooperative launch of as
+// Both sweeps through k_trsv_flow (kf_flow_fits): one cooperative launch of as
 // many CTAs as are resident at once, or as the chunks fill.  b and x in the
 // mesh's numbering whatever the pattern's.
 template <typename T> static void sptrsv_flow(DevMesh &m, const double *b, double *x)
@@ -3184,7 +3176,7 @@ template <typename T> static void sptrsv_flow(DevMesh &m, const double *b, doubl
 // false (nothing done) when the active schedule is not the packed one.
 bool sptrsv_permuted(DevMesh &m, const double *b, double *x, int precision)
 {
-  if (m.row_node && flow_fits(m)) {
+  if (m.row_node && kf_flow_fits(m)) {
     if (precision == 0) sptrsv_flow<double>(m, b, x);
     else sptrsv_flow<float>(m, b, x);
     return true;
@@ -3233,7 +3225,7 @@ void sptrsv(DevMesh &m, const double *b, double *x, int precision)
 {
   // (the other schedules run in the pattern's own numbering: a renumbered
   // pattern's data-flow sweeps are sptrsv_permuted's)
-  if (!m.row_node && flow_fits(m)) {
+  if (!m.row_node && kf_flow_fits(m)) {
     if (precision == 0) sptrsv_flow<double>(m, b, x);
     else sptrsv_flow<float>(m, b, x);
     return;
@@ -3406,7 +3398,7 @@ void sptrsv(DevMesh &m, const double *b, double *x, int precision)
 // here), for the allocation-free entry point in noalloc.cu.
 void sptrsv_flags(DevMesh &m, const double *b, double *x, int precision, uint32_t *flags)
 {
-  if (!m.row_node && flow_fits(m)) {
+  if (!m.row_node && kf_flow_fits(m)) {
     if (precision == 0) sptrsv_flow<double>(m, b, x);
     else sptrsv_flow<float>(m, b, x);
     return;

@@ -1,8 +1,8 @@
 """The data-flow triangular sweeps (the default schedule): both sweeps in one
 launch, every row waiting for the values it reads.
 
-Bit for bit the level launches' results (KFUN3D_SPTRSV=levels, the reference's
-arithmetic per row) at the sizes where the chunking can go wrong: fewer rows
+Bit for bit the level launches' results (KFUN3D_SPTRSV=pdl4, the reference's
+arithmetic per row, in both elimination orders) at the sizes where the chunking can go wrong: fewer rows
 than a warp takes, chunks that end inside a level, eight lanes a row and (from
 150,000 rows) four; several solves in a row, which alternate between the two
 solution buffers; right-hand sides with NaN and infinities, whose bits are also
@@ -46,7 +46,7 @@ def test_flow_sweeps_equal_level_launches(box_mesh, monkeypatch, n):
     res = {}
     for sched in ("flow", "levels"):
         if sched == "levels":
-            monkeypatch.setenv("KFUN3D_SPTRSV", "levels")
+            monkeypatch.setenv("KFUN3D_SPTRSV", "pdl4")
         m = kf.Mesh(path)
         v = m.view
         q = seeded_state(v.q.copy(), 41)
@@ -57,6 +57,7 @@ def test_flow_sweeps_equal_level_launches(box_mesh, monkeypatch, n):
                 kf.set_precision(prec)
                 m.fill(q, cdt)
                 m.ilu()
+                assert m.query("sptrsv_flow") == (sched == "flow"), (sched, order)
                 res[sched, order, prec] = [m.sptrsv(b) for b in right_hand_sides(v.dofs)]
                 assert kf.last_status() == 0, (sched, order, prec, kf.last_error())
         m.close()
