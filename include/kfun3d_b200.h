@@ -298,6 +298,17 @@ void kfun3d_device_release(GEOMETRY *g);
    in the reference. */
 int kfun3d_check_bounded_wait(void);
 
+/* One Gram-Schmidt step of the solver's GMRES in the current mode, for tests:
+   V holds k + 2 host vectors of 4*nnodes doubles one after the other (k from 0
+   to 29); vector k + 1 is orthogonalised against vectors 0 .. k
+   (src/kernel.c:129-141), normalised and written back, its coefficients and
+   norm go to h[0 .. k+1].  Fast mode also keeps the products of vector k with
+   those before it for the steps that follow, so a step on vectors of the
+   caller's own is reached through steps 0 .. k-1 on the same ones.  Returns
+   KFUN3D_OK or an error code (also recorded).  No counterpart in the
+   reference. */
+int kfun3d_gram_schmidt(const GEOMETRY *g, int k, double *V, double *h);
+
 /* Which device paths g's mirror uses (for tests and reports; builds the
    mirror on first use): key "sptrsv_schedule" -> the triangular-solve
    schedule of the active ILU(0) order (8 the packed factor: both sweeps in one

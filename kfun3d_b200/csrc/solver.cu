@@ -1779,6 +1779,22 @@ extern "C" double kfun3d_time_kernel(GEOMETRY *g, int which, int reps)
   return (double)ms / reps;
 }
 
+extern "C" int kfun3d_gram_schmidt(const GEOMETRY *g, int k, double *V, double *h)
+{
+  if (k < 0 || k > KF_NBASIS - 2 || !V || !h) {
+    kf_set_error(KFUN3D_ERR_ARG, "kfun3d_gram_schmidt: bad arguments");
+    return KFUN3D_ERR_ARG;
+  }
+  DevMesh *m = dev_or_fail(g);
+  if (!m) return kfun3d_gpu_last_status();
+  const size_t n = 4 * (size_t)m->N;
+  h2d(*m, m->V, V, (k + 2) * n);
+  orthogonalize(*m, ops(), k);
+  d2h(*m, V + (k + 1) * n, Vb(*m, k + 1), n);
+  d2h(*m, h, m->scal, k + 2);
+  return finish(*m, "kfun3d_gram_schmidt") ? KFUN3D_OK : kfun3d_gpu_last_status();
+}
+
 extern "C" int kfun3d_check_bounded_wait(void)
 {
   int ndev = 0;
