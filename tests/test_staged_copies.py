@@ -1,9 +1,11 @@
 """Large host arrays go to and from the device through pinned buffers filled by
 several threads; arrays that are pinned already are copied directly.  The same
 residual and gradients bit for bit either way, on calls in a row (the buffers
-are used again), with a last chunk that is not full.
+are used again), with last chunks that are not full.
 
-Sizes: 34 (5 MB out, copied directly), 66 (37 MB out, staged).
+Sizes: 34 (1 MB in and 5 MB out, both copied directly), 66 (9 MB in directly,
+37 MB out staged), 102 (34 MB in, 136 MB out, both staged: each call's copies
+out take the buffers that its copies in may still be leaving).
 """
 import ctypes as C
 
@@ -18,7 +20,7 @@ from kfun3d_b200 import api
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [34, 66])
+@pytest.mark.parametrize("n", [34, 66, 102])
 def test_pageable_arrays_equal_pinned_ones(box_mesh, n):
     kf.set_mode("fast")
     try:
