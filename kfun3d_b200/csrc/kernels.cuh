@@ -298,23 +298,41 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
 
 constexpr uint32_t KF_MBAR_LIMIT = 1u << 24;
 
+// One poll of phase `phase` of the mbarrier.
+__device__ __forceinline__ bool mbar_poll(unsigned a, unsigned phase)
+{
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(a), "r"(phase)
+      : "memory");
+  return done != 0;
+}
+
 // Bounded wait for phase `phase` of the mbarrier; false (and *err set) if it
-// gave up.  It gives up in two steps of `limit` polls: after the first *err is
-// set, in the second the copies may still land, so that a CTA does not return
-// while they are on their way into its shared memory.
-__device__ __forceinline__ bool mbar_wait(uint64_t *mbar, unsigned phase, int *err, uint32_t limit = KF_MBAR_LIMIT)
+// gave up.  The copies may then still be on their way: mbar_drain before the
+// CTA returns.
+__device__ __forceinline__ bool mbar_try(uint64_t *mbar, unsigned phase, int *err, uint32_t limit = KF_MBAR_LIMIT)
 {
   const unsigned a = smem_addr(mbar);
-  for (uint32_t spins = 0; spins < 2 * limit; spins++) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(phase)
-        : "memory");
-    if (done) return spins < limit;
-    if (spins == limit - 1) atomicExch(err, 1);
-  }
+  for (uint32_t spins = 0; spins < limit; spins++)
+    if (mbar_poll(a, phase)) return true;
+  atomicExch(err, 1);
+  return false;
+}
+
+// Sees out copies that a wait gave up on, bounded as that was.
+__device__ __forceinline__ void mbar_drain(uint64_t *mbar, unsigned phase, uint32_t limit = KF_MBAR_LIMIT)
+{
+  const unsigned a = smem_addr(mbar);
+  for (uint32_t spins = 0; spins < limit && !mbar_poll(a, phase); spins++) {}
+}
+
+__device__ __forceinline__ bool mbar_wait(uint64_t *mbar, unsigned phase, int *err, uint32_t limit = KF_MBAR_LIMIT)
+{
+  if (mbar_try(mbar, phase, err, limit)) return true;
+  mbar_drain(mbar, phase, limit);
   return false;
 }
 
@@ -2588,11 +2606,7 @@ __global__ void __launch_bounds__(128, MINB)
     const size_t own = 4 * (size_t)s0.x + r;
     double xi = 0.0;
     if (active && !upper) xi = b[4 * (size_t)s0.w + r];
-    if (!__all_sync(0xffffffffu, mbar_wait(&mbars[warp][st], phase, err))) {
-      // the other stage's copies, issued for the chunk after this one, land first
-      if (c + W < total) mbar_wait(&mbars[warp][st ^ 1], phase ^ (uint32_t)st, err);
-      break;
-    }
+    if (!__all_sync(0xffffffffu, mbar_try(&mbars[warp][st], phase, err))) break;
     const unsigned char *sg = stage0 + (size_t)st * stage_bytes;
     const T *sa = reinterpret_cast<const T *>(sg) + 4 * r;
     const uint32_t *sc = reinterpret_cast<const uint32_t *>(sg + (size_t)stage_blk * 16 * sizeof(T)) + (d0.z & 3u);
@@ -2693,6 +2707,10 @@ __global__ void __launch_bounds__(128, MINB)
     s1 = slot_of(c + 2 * W, dn);
     st ^= 1;
     if (st == 0) phase ^= 1;
+  }
+  if (c < total) {   // a chunk's copies did not come: no copy of either stage is left on its way
+    mbar_drain(&mbars[warp][st], phase);
+    if (c + W < total) mbar_drain(&mbars[warp][st ^ 1], phase ^ (uint32_t)st);
   }
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(ctl + 1, 1u) == gridDim.x - 1) {
