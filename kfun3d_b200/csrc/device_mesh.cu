@@ -325,7 +325,8 @@ void kf_free_packed(PackedSweep pk[2])
 // Each level's slots are cut into chunks three times: at most 32 rows and 256
 // blocks, at most 64 rows and 512 blocks (one CTA each), and for the
 // data-flow sweeps 4 rows and 40 blocks (8 lanes a row) or 8 rows and 64
-// blocks (4 lanes; one warp each).  KFUN3D_ERR_ARG (and nothing allocated) when a row has more than KF_PK_ROW_MAX blocks.
+// blocks (4 lanes; one warp each).  KFUN3D_ERR_ARG (and nothing allocated) when
+// a row has more than KF_PK_ROW_MAX blocks.
 // (f(i) for every i in [0, n), interleaved over the host's threads: for
 // items of uneven size, such as levels)
 template <class F> static void parallel_items(size_t n, size_t work, F f)
@@ -437,11 +438,13 @@ static void release_device(MatrixHandle *h)
   for (void *p : {m->pk_buf, (void *)m->flow_buf, (void *)m->flow_ctl})
     if (p) cudaFree(p);
   void *ptrs[] = {m->col, m->egeo, m->xyz, m->inc_ptr, m->inc_oth, m->inc_edge, m->inc_blk, m->inc_w, m->wf_nodes,
-                  m->wf_n, m->s_n, m->f_n, m->bnd_of, m->bndp, m->f_node, m->fres, m->bnd_node, m->bnd_ptr, m->bnd_ent, m->ia, m->ja,
-                  m->diag, m->tblk, m->lpos, m->last_lower, m->lev_l, m->lev_u, m->A, m->lslot, m->dinv,
+                  m->wf_n, m->s_n, m->f_n, m->bnd_of, m->bndp, m->f_node, m->fres, m->bnd_node, m->bnd_ptr, m->bnd_ent,
+                  m->ia, m->ja, m->diag, m->tblk, m->lpos, m->last_lower, m->lev_l, m->lev_u, m->A, m->lslot, m->dinv,
                   m->Af, m->dinvf, m->q, m->r, m->gx, m->gy, m->gz, m->cdt, m->w, m->t, m->x, m->rhs, m->V,
                   m->red, m->scal, m->forces, m->dscr, m->status, m->flags, m->gs_part, m->gs_seq_d, m->lsq_coef,
-                  m->qv, m->xyzv, m->rec, m->inc_othv, m->n0v, m->n1v, m->inc_geo, m->desc_l, m->desc_u, m->eoff, m->n1, m->in1_ptr, m->in1_edge, m->eres, m->n0s, m->pair_ptr, m->pairs, m->lev_ptr_d, m->bar, m->Z, m->qold, m->fy, m->fx, m->pscr, m->ord, m->rowof, m->egeo_s, m->sub_part};
+                  m->qv, m->xyzv, m->rec, m->inc_othv, m->n0v, m->n1v, m->inc_geo, m->desc_l, m->desc_u, m->eoff,
+                  m->n1, m->in1_ptr, m->in1_edge, m->eres, m->n0s, m->pair_ptr, m->pairs, m->lev_ptr_d, m->bar, m->Z,
+                  m->qold, m->fy, m->fx, m->pscr, m->ord, m->rowof, m->egeo_s, m->sub_part};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (m->h_scal) cudaFreeHost(m->h_scal);

@@ -402,7 +402,8 @@ struct DevMesh {
   // values they read instead of for levels
   bool pk_flow = true;            // used by mode 8 where the rows fit (KFUN3D_SPTRSV=packed: level launches)
   int flow_lanes = 8;             // lanes per row in the data-flow sweeps (4 or 8)
-  double *flow_buf = nullptr;     // [3][4N] y of the lower sweep, x of this and of the next solve (KF_FLOW_EMPTY where not written)
+  double *flow_buf = nullptr;     // [3][4N] y of the lower sweep, x of this and of the next solve (KF_FLOW_EMPTY
+                                  // where not written)
   unsigned *flow_ctl = nullptr;   // [0] which x buffer the next solve writes, [1] CTAs done
   int ilu_active = 0;             // 1: the spatial set is active
   uint32_t *ilu_rank = nullptr;   // [N] row of each node in the spatial set

@@ -737,11 +737,13 @@ __global__ void __launch_bounds__(128) k_residual(uint32_t N, const uint32_t *__
 // all four edges, and a 4 x 4 transpose inside the quad gives each lane its own
 // edge's state.  With a lane reading the state and the gradients of its own
 // edge's ends, each in a request of its own, the L1 data path was 75 % busy and
-// bounded the kernel.  Edges and nodes at 70^3 142 -> 123 us, at 120^3 522 -> 515
-// (with the node pass of that time; there the 384 MB of edge fluxes, written once and read twice, take 173 us at
-// a copy's rate); seven CTAs an SM (at 120^3 six take 550 us, five 581, eight 524
-// with the records loaded in two halves).
-// (not inlined: its registers are not the edges')
+// bounded the kernel.  Edges and nodes, with the node pass of that time, at 70^3
+// 142 -> 123 us, at 120^3 522 -> 515; seven CTAs an SM (at 120^3 six took 550 us,
+// five 581, eight 524 with the records loaded in two halves).  The edge fluxes
+// themselves, 384 MB written once and read twice at 120^3, take 173 us at a
+// copy's rate.
+//
+// farfield_store is not inlined: its registers are not the edges'.
 __device__ __noinline__ void farfield_store(double U, double V, const double *fn, const double4 *q, double4 *out)
 {
   *out = farfield_flux(U, V, fn[0], fn[1], fn[2], *q);
@@ -793,7 +795,9 @@ __global__ void __launch_bounds__(128, 7) k_flux_edges(uint32_t E, const uint32_
   } else {
     const int lane = threadIdx.x & 31, c = lane & 3, qb = lane & ~3;
 #if KF_FAST
-    const double hx = 0.5 * (xb.x - xa.x), hy = 0.5 * (xb.y - xa.y), hz = 0.5 * (xb.z - xa.z);   // to the midpoint
+    // to the midpoint, without the midpoint's own rounding (residual at 70^3
+    // against 80-bit arithmetic: 2.7e-15, with midpoint minus end point 3.1e-15)
+    const double hx = 0.5 * (xb.x - xa.x), hy = 0.5 * (xb.y - xa.y), hz = 0.5 * (xb.z - xa.z);
 #else
     const double xm = 0.5 * (xa.x + xb.x), ym = 0.5 * (xa.y + xb.y), zm = 0.5 * (xa.z + xb.z);
     const double hx = xm - xa.x, hy = ym - xa.y, hz = zm - xa.z, kx = xm - xb.x, ky = ym - xb.y, kz = zm - xb.z;
@@ -2795,7 +2799,8 @@ void gradient(DevMesh &m, const double *q)
     const uint32_t *ord = m.visit ? nullptr : m.ord, *oth = m.visit ? m.inc_othv : m.inc_oth;
     auto kern = m.rec_smem ? k_gradient_rec<true> : k_gradient_rec<false>;
     if (m.rec_smem) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.rec_smem);
-    kern<<<blocks(m.N, KF_GRAD_NODES), 4 * KF_GRAD_NODES, m.rec_smem, m.stream>>>(m.N, ord, m.inc_ptr, oth, m.inc_w, m.wstride, Q, m.rec, m.status + 1);
+    kern<<<blocks(m.N, KF_GRAD_NODES), 4 * KF_GRAD_NODES, m.rec_smem, m.stream>>>(
+        m.N, ord, m.inc_ptr, oth, m.inc_w, m.wstride, Q, m.rec, m.status + 1);
     kf_count_launch();
     return;
   }
@@ -2805,9 +2810,13 @@ void gradient(DevMesh &m, const double *q)
       cudaFuncSetAttribute(k_gradient_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       attr_set = true;
     }
-    k_gradient_tma<<<blocks(m.N, 128), 128, m.grad_smem, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride, (const double4 *)q, (double4 *)m.gx, (double4 *)m.gy, (double4 *)m.gz, m.status + 1);
+    k_gradient_tma<<<blocks(m.N, 128), 128, m.grad_smem, m.stream>>>(
+        m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride, (const double4 *)q, (double4 *)m.gx, (double4 *)m.gy,
+        (double4 *)m.gz, m.status + 1);
   } else {
-    k_gradient<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride, (const double4 *)q, (double4 *)m.gx, (double4 *)m.gy, (double4 *)m.gz);
+    k_gradient<<<blocks(m.N, 256), 256, 0, m.stream>>>(m.N, m.ord, m.inc_ptr, m.inc_oth, m.inc_w, m.wstride,
+                                                        (const double4 *)q, (double4 *)m.gx, (double4 *)m.gy,
+                                                        (double4 *)m.gz);
   }
   kf_count_launch();
 }
@@ -2836,11 +2845,13 @@ static void residual_or_jv(DevMesh &m, const double *q, double *r, int first_ord
     const uint32_t nfb = blocks(m.Nf, 128);
     const unsigned grid = m.E ? nfb + blocks(m.E, 128) : nfb;
     if (grid) {
-      (first_order ? k_flux_edges<true> : k_flux_edges<false>)<<<grid, 128, 0, m.stream>>>(m.E, E0, E1, m.egeo_s, X, Q, m.rec, m.eres, nfb, m.Nf, m.f_node, m.f_n, (const double4 *)q, u, v, m.fres);
+      (first_order ? k_flux_edges<true> : k_flux_edges<false>)<<<grid, 128, 0, m.stream>>>(
+          m.E, E0, E1, m.egeo_s, X, Q, m.rec, m.eres, nfb, m.Nf, m.f_node, m.f_n, (const double4 *)q, u, v, m.fres);
       kf_count_launch();
     }
     NodePass a{m.ord, m.in1_ptr, m.in1_edge, m.eoff, m.bndp, m.bnd_ptr, m.bnd_ent, m.wf_nodes, m.wf_n,
-               (const double *)m.fres, (const double4 *)q, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0};
+               (const double *)m.fres, (const double4 *)q, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+               0.0};
     if (jv) {
       a.jr = jv->r;
       a.jw = q;
@@ -3015,8 +3026,7 @@ void ilu(DevMesh &m, int precision)
       const cudaError_t e = cudaLaunchKernelExC(
           &cfg, precision == 0 ? (const void *)k_ilu_rows<double> : (const void *)k_ilu_rows<float>, args);
       if (e != cudaSuccess) kf_set_error(KFUN3D_ERR_CUDA, cudaGetErrorString(e));
-    } else
-    if (precision == 0 && m.pairs)
+    } else if (precision == 0 && m.pairs)
       k_ilu_level_pairs<<<blocks((size_t)nr * 16, 128), 128, 0, m.stream>>>(nr, m.lev_l + r0, m.ia, m.ja, m.diag,
                                                                             m.pair_ptr, m.pairs, m.lpos, m.A,
                                                                             m.lslot, m.dinv, status);

@@ -786,7 +786,7 @@ int kf_build_mesh_lists_device(DevMesh &m, const GEOMETRY *g)
     }
     // visit-order copies: each incidence's other end as a visit position and
     // its edge geometry, the edges' end points as visit positions, the
-    // coordinates in visit order, room for the state and the gradients
+    // coordinates in visit order, room for the state
     if (ok && m.visit) {
       ck(cudaMalloc(&m.inc_othv, (wst + 4) * sizeof(uint32_t)));   // padded, as inc_oth
       ck(cudaMemsetAsync(m.inc_othv, 0, (wst + 4) * sizeof(uint32_t), st));
@@ -794,8 +794,7 @@ int kf_build_mesh_lists_device(DevMesh &m, const GEOMETRY *g)
       ck(cudaMalloc(&m.n0v, E1 * sizeof(uint32_t)));
       ck(cudaMalloc(&m.n1v, E1 * sizeof(uint32_t)));
       ck(cudaMalloc(&m.xyzv, N1 * sizeof(double4)));
-      double4 **vv[] = {&m.qv};
-      for (double4 **v : vv) ck(cudaMalloc(v, N1 * sizeof(double4)));
+      ck(cudaMalloc(&m.qv, N1 * sizeof(double4)));
       if (ok) {
         if (E) {
           k_visit_incidence<<<nblk(ninc, 256), 256, 0, st>>>(ninc, m.inc_oth, m.inc_edge, m.rowof, m.egeo,

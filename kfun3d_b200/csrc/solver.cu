@@ -1385,12 +1385,17 @@ struct HostCopy {
 // buffers that several host threads fill (or empty) while the copies of the
 // others run: the driver's own path for pageable memory is one thread's memcpy
 // (about 5 GB/s into pages not yet touched; one residual of the 70^3 mesh, 11 MB
-// in and 44 MB out: 10.3 -> 5.2 ms).  To the host, the arrays are written when
-// the call returns; to the device, the copies are queued on the mesh's stream.
-// From 32 MB: shorter copies do not repay the threads' start (four calls that
-// copy 8 MB each way at 63^3: 5.9 ms staged, 5.5 directly).  The buffers (16 MB)
-// are the mesh's and go with it.  A chunk a
-// buffer, two buffers a thread; the threads take chunks in turn.
+// in, copied directly, and 44 MB out, staged: 9.8 -> 5.2 ms, on a state not passed
+// before 6.7 -> 5.0).  To the host, the arrays are written when the call returns;
+// to the device, the copies are queued on the mesh's stream.  A chunk a buffer,
+// two buffers a thread; the threads take chunks in turn.  The buffers (16 MB) are
+// the mesh's and go with it.
+// From 32 MB, where one array to the device breaks even; shorter copies do not
+// repay the threads' start.  A call directly / staged, one array to the device:
+// 8 MB 0.58 / 0.77 ms, 17 MB 1.09 / 1.29, 34 MB 2.03 / 2.03, 55 MB 3.7 / 2.65;
+// gradients and residual to the host, into pages not yet touched (and a quarter
+// as much to the device): 8 MB 1.45 / 1.52, 16 MB 2.67 / 2.76, 25 MB 3.80 / 3.42,
+// 34 MB 4.89 / 3.90, 44 MB 6.67 / 4.90.
 constexpr size_t STAGE_MIN = 32u << 20, STAGE_CHUNK = 1u << 20;
 
 bool stage_ready(DevMesh &m)
