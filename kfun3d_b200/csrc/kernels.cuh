@@ -2979,9 +2979,10 @@ static void pack_factor(DevMesh &m, int precision)
 }
 
 // Before sweeps over the packed copy: made again when it holds another
-// precision's or order's blocks, or when the matrix was filled after it.  (A
+// precision's or order's blocks, or when the FP64 matrix was filled after it (an
+// FP32 copy stays the last FP32 factor's until another takes its place).  A
 // solve factors, which packs, before it captures its steps: no captured graph
-// holds these launches.)
+// holds these launches.
 static void packed_current(DevMesh &m, int precision)
 {
   if (m.pk_precision != precision || m.pk_order != m.ilu_active) pack_factor(m, precision);
